@@ -75,7 +75,9 @@ enum xfb_ade_kind { XFB_ADE_NONE = 0, XFB_ADE_DEBYE = 1, XFB_ADE_DRUDE = 2, XFB_
  * separate launches per face (src/include/updator/update_scheme.cuh:132-197,
  * src/boundary/pml_corrector.cu:9-291,
  * src/waveform_source/tfsf/tfsf_corrector.cu:155-271); 3-D scenes without
- * dispersive media only.  AUTO: FUSED (3-D and 2-D TMz). */
+ * dispersive media only.  AUTO: FUSED (3-D and 2-D TMz), where 3-D scenes with
+ * a CPML are stepped by two in-place passes (H, then E) instead of the sweep,
+ * with the same results and the same checkpoints. */
 enum xfb_kernel_path { XFB_PATH_AUTO = 0, XFB_PATH_SPLIT = 1, XFB_PATH_FUSED = 2, XFB_PATH_PLAIN = 3 };
 
 #define XFB_MAX_POLES 4

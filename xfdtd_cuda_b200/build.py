@@ -31,8 +31,10 @@ def nvcc() -> str:
 
 
 # (source, fmad) pairs
-UNITS = [("api.cu", False), ("engine_f64.cu", False), ("engine_f32.cu", True), ("labc_train.cu", True),
-         ("scene_compile.cpp", False), ("core_ingest.cpp", False), ("host_copy.cpp", False)]
+UNITS = [("engine_f64.cu", False), ("batch_f64.cu", False), ("engine_f32.cu", True), ("batch_f32.cu", True),
+         ("api.cu", False), ("twopass_f64.cu", False), ("twopass_f32.cu", True), ("tb2d_f64.cu", False),
+         ("tb2d_f32.cu", True), ("labc_train.cu", True), ("scene_compile.cpp", False), ("core_ingest.cpp", False),
+         ("host_copy.cpp", False)]
 
 
 def sources() -> list[Path]:

@@ -153,7 +153,7 @@ long long roundup(long long v, long long m) { return (v + m - 1) / m * m; }
 bool fused(const xfb_handle* h) { return h->path == XFB_PATH_FUSED; }
 bool plain(const xfb_handle* h) { return h->path == XFB_PATH_PLAIN; }
 // field set holding the state after h->step steps
-int cur_set(const xfb_handle* h) { return fused(h) ? static_cast<int>(h->step & 1) : 0; }
+int cur_set(const xfb_handle* h) { return h->two_pass ? h->live : fused(h) ? static_cast<int>(h->step & 1) : 0; }
 void* field_ptr(const xfb_handle* h, int set, int q) { return set ? h->f1[q] : h->f[q]; }
 
 // element offset of component index (i, j, k) in the padded layout
@@ -180,8 +180,10 @@ int launches_per_step(const xfb_handle* h) {
     return 6 + 2 * faces + (c.tfsf_on ? 24 : 0) + (c.nf_on ? 1 : 0) + (c.td_on ? 2 : 0) + (c.probes.empty() ? 0 : 1) +
            static_cast<int>(c.movies.size());
   }
-  int bulk = 2;
-  if (fused(h)) {
+  int bulk = 2;  // H and E half-steps
+  if (h->two_pass) {
+    bulk += h->ade_deferred && h->n_ade_runs > 0 ? 1 : 0;  // k_tp_ade
+  } else if (fused(h)) {
     bulk = c.dim == 2 ? 1
                       : (h->n_step_items[step_tile_index(h->tj)] > 0 ? 1 : 0) + (h->ade_deferred ? 1 : 0) +
                             (h->lines_on ? 1 : 0);  // k_tfsf_lines
@@ -435,6 +437,7 @@ int xfb_set_kernel_path(xfb_handle* h, int path) {
   if (path < XFB_PATH_AUTO || path > XFB_PATH_PLAIN) return set_err(h, XFB_ERR_INVALID, "unknown kernel path");
   if (h->inited) return set_err(h, XFB_ERR_STATE, "set the kernel path before xfb_init");
   h->path = path;
+  h->path_auto = path == XFB_PATH_AUTO;
   return XFB_OK;
 }
 
@@ -507,6 +510,8 @@ int xfb_init(xfb_handle* h, long long total_steps) {
     return rc;
   }
   h->step = 0;
+  h->live = 0;
+  h->two_pass = h->c.prec == XFB_FP64 ? tp_plan<double>(h) : tp_plan<float>(h);
   h->inited = true;
   return XFB_OK;
 }
@@ -546,11 +551,28 @@ int xfb_sync(xfb_handle* h) {
   return step_status(h);
 }
 
+}  // extern "C"
+
+namespace xfb {
+int tp_leave(xfb_handle* h) {
+  if (!h->two_pass) return XFB_OK;
+  const int rc = h->c.prec == XFB_FP64 ? tp_normalise<double>(h) : tp_normalise<float>(h);
+  if (rc) return rc;
+  for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);  // the step's launch list changes
+  h->graphs.clear();
+  h->two_pass = false;
+  return XFB_OK;
+}
+}  // namespace xfb
+
+extern "C" {
+
 int xfb_set_wait_limit(xfb_handle* h, int polls) {
   int rc = check_handle(h, true);
   if (rc || (rc = not_batched(h))) return rc;
   if (polls < 0) return set_err(h, XFB_ERR_INVALID, "negative poll limit");
   if (!h->step_err) return set_err(h, XFB_ERR_STATE, "only the 3-D one-sweep step has bounded waits");
+  if ((rc = tp_leave(h))) return rc;  // the two-pass step has none
   return copy(h, h->step_err + 1, &polls, sizeof(int), cudaMemcpyHostToDevice);
 }
 
@@ -1028,6 +1050,8 @@ int xfb_get_state(xfb_handle* h, void* dst, size_t len) {
   if ((rc = xfb_state_size(h, &need))) return rc;
   if (!dst || len < need) return set_err(h, XFB_ERR_RANGE, "state buffer too small");
   if ((rc = nf2ff_flush(h))) return rc;  // the state holds accumulators, not the sample ring
+  // the state image is the one-sweep path's: the fields in set step & 1
+  if ((rc = h->c.prec == XFB_FP64 ? tp_normalise<double>(h) : tp_normalise<float>(h))) return rc;
   XFB_CUDA(h, cudaStreamSynchronize(h->stream));
   char* o = static_cast<char*>(dst);
   std::memcpy(o, &h->step, sizeof(long long));
@@ -1058,6 +1082,7 @@ int xfb_set_state(xfb_handle* h, const void* src, size_t len) {
       o += b.bytes;
     }
   h->step = step;
+  h->live = static_cast<int>(step & 1);
   return XFB_OK;
 }
 
@@ -1157,6 +1182,7 @@ int xfb_set_learned_abc(xfb_handle* h, const float* weights, int n_weights) {
     if ((rc = alloc(h, &p, 2 * labc_layout(h->c.nx, h->c.ny, h->c.nz).off[12] * sizeof(float), true))) return rc;
     h->labc_hist = static_cast<float*>(p);
   }
+  if ((rc = tp_leave(h))) return rc;
   if ((rc = copy(h, h->labc_w, wb.data(), wb.size() * sizeof(uint16_t), cudaMemcpyHostToDevice))) return rc;
   h->labc_on = true;
   return XFB_OK;
@@ -1239,6 +1265,7 @@ int xfb_batch_init(xfb_batch* b, long long total_steps) {
     int rc = xfb_init(h, total_steps);
     h->batch = b;
     if (rc) return batch_err(b, rc, "scene init failed: " + h->err);
+    h->two_pass = false;  // the batch's kernels alternate the field sets
     b->cells += static_cast<long long>(h->c.nx) * h->c.ny * h->c.nz;
   }
   if (cudaSetDevice(dev) != cudaSuccess) return batch_err(b, XFB_ERR_CUDA, "cudaSetDevice");

@@ -20,7 +20,6 @@
 #include "kernels.cuh"
 #include "labc.cuh"
 #include "plain.cuh"
-#include "tb2d.cuh"
 
 namespace xfb {
 
@@ -30,38 +29,14 @@ inline int upload_td(xfb_handle* h);
 template <typename T>
 int encode_stage_maps(xfb_handle* h);
 
-// Tile of the blocked 2-D step: TJ + 2 S + 1 columns fill a shared row of
-// kTbPitch, TI rows keep the tile count within two CTAs per SM when it can
-// and the tile's shared memory within a CTA's 227 KB.
-// False (one launch per step) when blocking is off, the scene has movie
-// monitors (recorded between steps), or a tile's region would hold more CPML
-// rows or columns than its psi tables.
+// Blocked 2-D step (tb2d_f32.cu, tb2d_f64.cu): its tile plan (false: one
+// launch per step), the kernel's one-time set-up, and one launch.
 template <typename T>
-bool tb2d_plan(xfb_handle* h) {
-  const Compiled& c = h->c;
-  const int S = h->tb_steps;
-  if (c.dim != 2 || S <= 0 || !c.movies.empty()) return false;
-  const int TJ = kTbPitch - 1 - 2 * S;
-  if (TJ < 16) return false;
-  const int ntj = (c.ny + TJ - 1) / TJ;
-  int TI = (c.nx + std::max(1, 296 / ntj) - 1) / std::max(1, 296 / ntj);
-  TI = std::min(64, std::max(16, TI));
-  // the tile's shared memory within the 227 KB a CTA may use
-  while (TI > 16 && TbLayout<T>(TI + 2 * S + 1, c.n_mat).bytes > 227u * 1024u) --TI;
-  if (TbLayout<T>(TI + 2 * S + 1, c.n_mat).bytes > 227u * 1024u) return false;
-  auto fits = [&](int n, int tile, int lo, int hi) {  // slab cells of every tile's region along one axis
-    for (int a0 = 0; a0 < n; a0 += tile) {
-      int cnt = 0;
-      for (int q = std::max(0, a0 - S); q <= std::min(n - 1, a0 + tile + S); ++q) cnt += (q < lo || q >= n - hi) ? 1 : 0;
-      if (cnt > kTbSlab) return false;
-    }
-    return true;
-  };
-  if (!fits(c.nx, TI, c.pml[0], c.pml[1]) || !fits(c.ny, TJ, c.pml[2], c.pml[3])) return false;
-  h->tb_ti = TI;
-  h->tb_tj = TJ;
-  return true;
-}
+bool tb2d_plan(xfb_handle* h);
+template <typename T>
+int tb2d_prepare(xfb_handle* h);
+template <typename T>
+void launch_tb2d(xfb_handle* h, int off, int S);
 
 // Update coefficients rounded to a 16-bit storage format (round to nearest
 // even) and widened back: what a LUT stored in that format would hold.
@@ -222,11 +197,7 @@ int init_device(xfb_handle* h) {
     if (h->tb_on) {  // the E-side psi alternates too on the blocked path
       if ((rc = alloc(h, &h->psi_e1[0], bx, true))) return rc;
       if ((rc = alloc(h, &h->psi_e1[1], by, true))) return rc;
-      // the kernel's shared-memory limit, set (and the kernel loaded) here,
-      // outside any stream capture of the step loop
-      const TbLayout<T> lay(h->tb_ti + 2 * h->tb_steps + 1, c.n_mat);
-      XFB_CUDA(h, cudaFuncSetAttribute(k_step2_tb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(lay.bytes)));
+      if ((rc = tb2d_prepare<T>(h))) return rc;
     }
   }
   // TFSF
@@ -985,7 +956,7 @@ void plain_pml(xfb_handle* h, const GridP<T>& g) {
 template <typename T>
 void enqueue_records(xfb_handle* h, int parity, TimeP tp, cudaStream_t s, Prof* pf) {
   const Compiled& c = h->c;
-  GridP<T> g = grid_params<T>(h, fused(h) ? 1 - parity : 0);
+  GridP<T> g = grid_params<T>(h, out_set(h, parity));
   if (c.nf_on) {
     NfP nf{};
     nf.nfreq = static_cast<int>(c.freqs.size());
@@ -1021,7 +992,7 @@ void enqueue_records(xfb_handle* h, int parity, TimeP tp, cudaStream_t s, Prof* 
     const long long per = static_cast<long long>(n0) * n1 * n2;
     const int blocks = static_cast<int>(std::min<long long>((per + 255) / 256, 1024));
     prof_begin(h, pf, XFB_K_MOVIE);
-    k_movie<T><<<blocks, 256, 0, s>>>(as<const T>(field_ptr(h, fused(h) ? 1 - parity : 0, mv.field)), h->sx, h->sy, mv.lo[0], mv.lo[1], mv.lo[2], n0, n1, n2,
+    k_movie<T><<<blocks, 256, 0, s>>>(as<const T>(field_ptr(h, out_set(h, parity), mv.field)), h->sx, h->sy, mv.lo[0], mv.lo[1], mv.lo[2], n0, n1, n2,
                                       mv.interval, h->movie_out[m], h->movie_frames[m], tp, own_lo(h), own_hi(h));
     prof_end(h, pf);
   }
@@ -1030,7 +1001,7 @@ void enqueue_records(xfb_handle* h, int parity, TimeP tp, cudaStream_t s, Prof* 
 template <typename T>
 void enqueue_update(xfb_handle* h, int off, Prof* pf);
 template <typename T>
-void launch_tb2d(xfb_handle* h, int off, int S);
+void tp_update(xfb_handle* h, TimeP tp, cudaStream_t st, Prof* pf);
 
 template <typename T>
 void enqueue_step(xfb_handle* h, int off, Prof* pf = nullptr) {
@@ -1046,7 +1017,7 @@ void enqueue_update(xfb_handle* h, int off, Prof* pf) {
   TimeP tp{h->t_dev, off};
   const int parity = static_cast<int>((h->step + off) & 1);
   // fields after this step: the written set (one-sweep) or the only set (split)
-  GridP<T> g = grid_params<T>(h, fused(h) ? 1 - parity : 0);
+  GridP<T> g = grid_params<T>(h, out_set(h, parity));
   PmlP<T> pm = pml_params<T>(h);
   TfsfP tf = tfsf_params(h);
   cudaStream_t s = h->stream;
@@ -1065,6 +1036,8 @@ void enqueue_update(xfb_handle* h, int off, Prof* pf) {
     if (c.tfsf_on) plain_tfsf<T>(h, g, tp, 0);
     plain_pml<T, true>(h, g);
     prof_end(h, pf);
+  } else if (h->two_pass) {
+    tp_update<T>(h, tp, s, pf);
   } else if (fused(h)) {
     if (c.dim == 3 && h->lines_on) {  // the TFSF line values this step's kernel stages
       prof_begin(h, pf, XFB_K_AUX);
@@ -1144,23 +1117,6 @@ int slab_record(xfb_handle* h) {
   return XFB_OK;
 }
 
-// One blocked 2-D launch: steps [off, off + S) of the chunk (S odd), read
-// set and E-side psi buffer (step & 1), write the others.
-template <typename T>
-void launch_tb2d(xfb_handle* h, int off, int S) {
-  const Compiled& c = h->c;
-  const int parity = static_cast<int>((h->step + off) & 1);
-  const TbLayout<T> lay(h->tb_ti + 2 * S + 1, c.n_mat);
-  T* ez_x[2] = {as<T>(h->psi[1]), as<T>(h->psi_e1[0])};
-  T* ez_y[2] = {as<T>(h->psi[2]), as<T>(h->psi_e1[1])};
-  ProbeP pr{static_cast<int>(c.probes.size()), h->probe_idx, h->probe_field, h->probe_out, c.total_steps};
-  const dim3 grid((c.ny + h->tb_tj - 1) / h->tb_tj, (c.nx + h->tb_ti - 1) / h->tb_ti);
-  k_step2_tb<T><<<grid, kTbThreads, lay.bytes, h->stream>>>(
-      grid_params<T>(h, parity), grid_params<T>(h, 1 - parity), pml_params<T>(h), psi_h_set<T>(h, parity),
-      psi_h_set<T>(h, 1 - parity), ez_x[parity], ez_y[parity], ez_x[1 - parity], ez_y[1 - parity], tfsf_params(h),
-      TimeP{h->t_dev, off}, pr, S, h->tb_ti, h->tb_tj, c.n_mat, h->scratch_err);
-}
-
 template <typename T>
 void enqueue_chunk(xfb_handle* h, int n) {
   if (h->tb_on) {  // blocked 2-D: launches of odd step counts (each flips the sets once)
@@ -1185,7 +1141,7 @@ int run_steps(xfb_handle* h, long long n) {
   while (left > 0) {
     const int chunk = static_cast<int>(std::min<long long>(left, h->graph_steps));
     if (h->graph_on) {
-      const int key = chunk * 2 + static_cast<int>(h->step & 1);
+      const int key = chunk * 2 + (h->two_pass ? h->live : static_cast<int>(h->step & 1));
       auto it = h->graphs.find(key);
       if (it == h->graphs.end()) {
         cudaGraph_t graph;
@@ -1766,6 +1722,10 @@ int batch_run(xfb_batch* b, long long n) {
   template int read_bytes_t<T>(xfb_handle*, void*, const void*, size_t);                   \
   template int write_field_t<T>(xfb_handle*, int, const double*);                          \
   template void launch_nonfinite<T>(xfb_handle*);                                          \
+  }
+
+#define XFB_INSTANTIATE_BATCH(T)                                                           \
+  namespace xfb {                                                                          \
   template int batch_init<T>(xfb_batch*);                                                  \
   template int batch_run<T>(xfb_batch*, long long);                                        \
   }

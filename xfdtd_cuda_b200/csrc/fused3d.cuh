@@ -291,6 +291,30 @@ __device__ __forceinline__ C4<double> ld_c4(const double* p) {
   return {a.x, a.y, b.x, b.y};
 }
 
+// V consecutive values of one row, moved by one 16-byte access.
+template <typename T>
+struct Vec16;
+template <>
+struct Vec16<float> {
+  static constexpr int V = 4;
+  float a[4];
+  __device__ __forceinline__ void ld(const void* p) {
+    const float4 v = *static_cast<const float4*>(p);
+    a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+  }
+  __device__ __forceinline__ void st(void* p) const { *static_cast<float4*>(p) = make_float4(a[0], a[1], a[2], a[3]); }
+};
+template <>
+struct Vec16<double> {
+  static constexpr int V = 2;
+  double a[2];
+  __device__ __forceinline__ void ld(const void* p) {
+    const double2 v = *static_cast<const double2*>(p);
+    a[0] = v.x; a[1] = v.y;
+  }
+  __device__ __forceinline__ void st(void* p) const { *static_cast<double2*>(p) = make_double2(a[0], a[1]); }
+};
+
 // Geometry and shared-memory layout of k_step3 (dynamic shared memory).
 template <typename T, int R, int NWM, int NS_>
 struct StepCfg {

@@ -43,6 +43,11 @@ struct xfb_handle {
   unsigned hint_grid[3] = {1, 1, 1}, hint_block[3] = {1, 1, 1};
   int tk = 32, tj = 16;
   int path = XFB_PATH_AUTO;  // resolved at init: XFB_PATH_SPLIT or XFB_PATH_FUSED
+  bool path_auto = true;     // the path was left to the library
+  // two-pass 3-D step (twopass.cuh): steps in place on field set `live` (0 or
+  // 1) instead of alternating between the sets; the automatic path only
+  bool two_pass = false;
+  int live = 0;
   int graph_on = 1, graph_steps = 64;
   int coeff_storage = XFB_COEFF_NATIVE;  // rounding of the update-coefficient LUT (xfb_set_coeff_storage)
   // 2-D temporal blocking (k_step2_tb): steps per launch (odd; 0: one launch
@@ -249,6 +254,8 @@ inline int own_hi(const xfb_handle* h) {
   return is_slab(h) && h->slab_i1 < h->c.nx ? h->slab_i1 : h->c.nx + 1;
 }
 int cur_set(const xfb_handle* h);
+// field set the step that reads set `parity` leaves its result in
+inline int out_set(const xfb_handle* h, int parity) { return h->two_pass ? h->live : fused(h) ? 1 - parity : 0; }
 void* field_ptr(const xfb_handle* h, int set, int q);
 long long off3(const xfb_handle* h, int i, int j, int k);
 void comp_shape(const Compiled& c, int f, int s[3]);
@@ -266,6 +273,12 @@ template <typename T> int read_field_t(xfb_handle* h, int f, double* dst);
 template <typename T> int read_bytes_t(xfb_handle* h, void* dst, const void* src, size_t bytes);
 template <typename T> int write_field_t(xfb_handle* h, int f, const double* src);
 template <typename T> void launch_nonfinite(xfb_handle* h);
+// two-pass 3-D step (twopass_f32.cu, twopass_f64.cu)
+template <typename T> bool tp_plan(const xfb_handle* h);
+template <typename T> int tp_normalise(xfb_handle* h);
+// Back to the one-sweep kernels from the current state (monitor reads, state
+// and results are unaffected).
+int tp_leave(xfb_handle* h);
 template <typename T> int batch_init(xfb_batch* b);
 template <typename T> int batch_run(xfb_batch* b, long long n);
 void batch_free(xfb_batch* b);

@@ -139,6 +139,35 @@ __device__ __forceinline__ void add_inc(T& f, double inc, double coef) {
 }
 
 // ---------------------------------------------------------------------------
+// The update terms with their rounding spelled out, for kernels whose FP32
+// results must not depend on how the compiler contracts an expression: FP32
+// fuses where the one-sweep bodies' code does (so every 3-D path rounds alike),
+// FP64 rounds every operation, in the reference's order.
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mad(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+// c h + p dp - q dq
+template <typename T>
+__device__ __forceinline__ T h_next(T c, T h, T p, T dp, T q, T dq) {
+  return mad(-q, dq, mad(p, dp, mul(c, h)));
+}
+// c e - p dp + q dq
+template <typename T>
+__device__ __forceinline__ T e_next(T c, T e, T p, T dp, T q, T dq) {
+  return mad(q, dq, mad(c, e, -mul(p, dp)));
+}
+// b psi + a d: the x slabs, and the y and z slabs
+template <typename T>
+__device__ __forceinline__ T psi_next_x(T b, T psi, T a, T d) {
+  return mad(a, d, mul(b, psi));
+}
+template <typename T>
+__device__ __forceinline__ T psi_next_yz(T b, T psi, T a, T d) {
+  return mad(b, psi, mul(a, d));
+}
+
+// ---------------------------------------------------------------------------
 // CPML slab lookup: slab plane index of coordinate q on an axis with N/P
 // layers Ln/Lp and n cells, or -1.
 __device__ __forceinline__ int slab(int q, int n, int Ln, int Lp) {
@@ -307,21 +336,20 @@ __device__ __forceinline__ T ade_e(const AdeP<T>& a, int comp, long long bi, int
 // overlap; the arithmetic and its order are those of ade_e.  Valid only when
 // no dispersive cell also takes a TFSF or CPML correction, which the
 // reference applies after the ADE update.
+// ADE update of one dispersive cell of the box: E^n in `ec`, the plain eNext
+// values in `pl`, E^{n+1} to `d`.
 template <typename T>
-__device__ __forceinline__ void ade_box_cell(const GridP<T>& s, const GridP<T>& d, const AdeP<T>& ad, int i, int j,
-                                             int k, long long idx, int m) {
+__device__ __forceinline__ void ade_cell(const GridP<T>& d, const AdeP<T>& ad, int i, int j, int k, long long idx,
+                                         int m, const T (&ec)[3], const T (&pl)[3]) {
   constexpr int MP = 4;  // XFB_MAX_POLES
   const long long bi = static_cast<long long>(i - ad.b0) * ad.bsx + static_cast<long long>(j - ad.b2) * ad.bsy + (k - ad.b4);
   const bool upd[3] = {j > 0 && k > 0, i > 0 && k > 0, i > 0 && j > 0};
   T* dd[3] = {d.ex, d.ey, d.ez};
-  const T* ss[3] = {s.ex, s.ey, s.ez};
   const bool ml = ad.kind == kAdeMLorentz;
   const int P = ad.P;
-  T ec[3], pl[3], J[3][MP], Jp[3][MP], Ep[3];
+  T J[3][MP], Jp[3][MP], Ep[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    ec[c] = ss[c][idx];
-    pl[c] = dd[c][idx];
     Ep[c] = ml ? ad.Ep[c * ad.bn + bi] : T(0);
 #pragma unroll
     for (int p = 0; p < MP; ++p) {
@@ -368,6 +396,14 @@ __device__ __forceinline__ void ade_box_cell(const GridP<T>& s, const GridP<T>& 
     }
     dd[c][idx] = e_new;
   }
+}
+
+// The cell after a one-sweep step: the plain values are in `d`, E^n in `s`.
+template <typename T>
+__device__ __forceinline__ void ade_box_cell(const GridP<T>& s, const GridP<T>& d, const AdeP<T>& ad, int i, int j,
+                                             int k, long long idx, int m) {
+  const T ec[3] = {s.ex[idx], s.ey[idx], s.ez[idx]}, pl[3] = {d.ex[idx], d.ey[idx], d.ez[idx]};
+  ade_cell(d, ad, i, j, k, idx, m, ec, pl);
 }
 
 template <typename T>
