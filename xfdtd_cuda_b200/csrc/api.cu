@@ -794,6 +794,13 @@ int xfb_read_nf2ff_all(xfb_handle* h, int freq, double* dst, size_t len, long lo
                                : read_bytes_t<float>(h, dst, src, n * sizeof(double2));
 }
 
+// The far-field integral of n directions; the kernel writes all 4 outputs of
+// every direction.
+static void launch_far(const FarP& fp, int n, cudaStream_t s) {
+  if (n >= kFarManyMin) k_far_many<<<(n + 31) / 32, 32 * kFarWarps, 0, s>>>(fp, n);
+  else k_far<<<n, 256, 0, s>>>(fp);
+}
+
 int xfb_far_field(xfb_handle* h, int freq, int n, const double* theta, const double* phi, double* out) {
   int rc = check_handle(h, true);
   if (rc) return rc;
@@ -830,7 +837,7 @@ int xfb_far_field(xfb_handle* h, int freq, int n, const double* theta, const dou
   fp.k = 2 * kPi * c.freqs[freq] / c0();
   fp.eta = std::sqrt(kMu0 / kEps0);
   fp.theta = d_th; fp.phi = d_ph; fp.out = d_out;
-  k_far<<<n, 256, 0, h->stream>>>(fp);
+  launch_far(fp, n, h->stream);
   XFB_CUDA(h, cudaGetLastError());
   XFB_CUDA(h, cudaMemcpyAsync(out, d_out, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   XFB_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -868,7 +875,7 @@ int xfb_far_field_static(xfb_handle* h, int freq, int n, const double* theta, co
   fp.k = 2 * kPi * c.freqs[freq] / c0();
   fp.eta = std::sqrt(kMu0 / kEps0);
   fp.theta = d_th; fp.phi = d_ph; fp.out = d_out;  // k_far writes all 4 outputs of every angle
-  k_far<<<n, 256, 0, h->stream>>>(fp);
+  launch_far(fp, n, h->stream);
   XFB_CUDA(h, cudaGetLastError());
   XFB_CUDA(h, cudaMemcpyAsync(out, d_out, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   XFB_CUDA(h, cudaStreamSynchronize(h->stream));
