@@ -271,10 +271,11 @@ int xfb_set_kernel_path(xfb_handle* h, int path);
 
 /* 2-D TMz scenes on the one-sweep path: steps advanced per launch by the
  * temporally blocked kernel (each CTA advances its tile plus a halo of that
- * many cells in shared memory and records its probes every step), odd, at
- * most 31; default 9; 0 launches once per step.  Scenes with movie monitors
- * or CPML slabs wider than a tile's psi tables step once per launch.  Results
- * are identical either way.  Before xfb_init. */
+ * many cells in registers and records its probes every step), odd, at most 31;
+ * by default the library chooses (up to 11); 0 launches once per step.  Scenes
+ * with movie monitors, or whose tiles do not fit a CTA's shared memory at that
+ * many steps, step once per launch.  Results are identical either way.  Before
+ * xfb_init. */
 int xfb_set_temporal_block(xfb_handle* h, int steps);
 
 /* Storage trial of the update coefficients, no counterpart in the reference

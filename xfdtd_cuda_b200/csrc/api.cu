@@ -447,6 +447,7 @@ int xfb_set_temporal_block(xfb_handle* h, int steps) {
     return set_err(h, XFB_ERR_INVALID, "steps per launch must be 0 (off) or odd, at most 31");
   if (h->inited) return set_err(h, XFB_ERR_STATE, "set the temporal blocking before xfb_init");
   h->tb_steps = steps;
+  h->tb_given = true;
   return XFB_OK;
 }
 

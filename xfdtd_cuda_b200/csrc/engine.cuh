@@ -37,6 +37,8 @@ template <typename T>
 int tb2d_prepare(xfb_handle* h);
 template <typename T>
 void launch_tb2d(xfb_handle* h, int off, int S);
+template <typename T>
+void tb2d_chunk(xfb_handle* h, int n);
 
 // Update coefficients rounded to a 16-bit storage format (round to nearest
 // even) and widened back: what a LUT stored in that format would hold.
@@ -1119,13 +1121,8 @@ int slab_record(xfb_handle* h) {
 
 template <typename T>
 void enqueue_chunk(xfb_handle* h, int n) {
-  if (h->tb_on) {  // blocked 2-D: launches of odd step counts (each flips the sets once)
-    for (int off = 0; off < n;) {
-      int S = std::min(h->tb_steps, n - off);
-      if (S % 2 == 0) --S;
-      launch_tb2d<T>(h, off, S);
-      off += S;
-    }
+  if (h->tb_on) {
+    tb2d_chunk<T>(h, n);
   } else {
     for (int s = 0; s < n; ++s) enqueue_step<T>(h, s);
   }

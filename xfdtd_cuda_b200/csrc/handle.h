@@ -51,11 +51,11 @@ struct xfb_handle {
   int graph_on = 1, graph_steps = 64;
   int coeff_storage = XFB_COEFF_NATIVE;  // rounding of the update-coefficient LUT (xfb_set_coeff_storage)
   // 2-D temporal blocking (k_step2_tb): steps per launch (odd; 0: one launch
-  // per step), whether init enabled it, the tile rows / columns, and the
-  // second set of the E-side psi (ez_x, ez_y) it alternates with psi[1], psi[2]
+  // per step), whether init enabled it, its plan, and the second set of the E-side psi (ez_x, ez_y) it alternates with psi[1], psi[2]
   int tb_steps = 9;
+  bool tb_given = false;  // tb_steps set by the caller, else the plan chooses
   bool tb_on = false;
-  int tb_ti = 0, tb_tj = 0;
+  int tb_warps = 0, tb_max = 0;  // the plan: warps of a CTA, steps of a launch at most
   void* psi_e1[2] = {};
   std::map<int, cudaGraphExec_t> graphs;
   std::vector<Buf> bufs;

@@ -157,7 +157,7 @@ template <typename T>
 __device__ __forceinline__ T e_next(T c, T e, T p, T dp, T q, T dq) {
   return mad(q, dq, mad(c, e, -mul(p, dp)));
 }
-// b psi + a d: the x slabs, and the y and z slabs
+// b psi + a d: the x slabs, and the y and z slabs (in 2-D all)
 template <typename T>
 __device__ __forceinline__ T psi_next_x(T b, T psi, T a, T d) {
   return mad(a, d, mul(b, psi));

@@ -7,46 +7,107 @@
 
 namespace xfb {
 
-// Tile of the blocked 2-D step: TJ + 2 S + 1 columns fill a shared row of
-// kTbPitch, TI rows keep the tile count within two CTAs per SM when it can
-// and the tile's shared memory within a CTA's 227 KB.
-// False (one launch per step) when blocking is off, the scene has movie
-// monitors (recorded between steps), or a tile's region would hold more CPML
-// rows or columns than its psi tables.
+// Shared-memory limit of a CTA.
+constexpr size_t kTbSmem = 227u * 1024u;
+
+// Largest CPML slab row and lane-block counts of any tile's region.
 template <typename T>
-bool tb2d_plan(xfb_handle* h) {
+void tb2d_slabs(const Compiled& c, int nw, int S, int& nsx, int& nsy) {
+  const TbGeom<T> g(nw, S);
+  nsx = nsy = 0;
+  for (int i0 = 0; i0 < c.nx; i0 += g.ti) nsx = std::max(nsx, TbSlab(i0 - S, g.xi, c.nx, c.pml[0], c.pml[1]).count());
+  for (int j0 = 0; j0 < c.ny; j0 += g.tj)
+    nsy = std::max(nsy, TbBlocks(TbSlab(j0 - g.hl, kTbCols, c.ny, c.pml[2], c.pml[3]), j0 - g.hl).count());
+}
+
+template <typename T>
+size_t tb2d_bytes(const Compiled& c, int nw, int S, int& nsx, int& nsy) {
+  tb2d_slabs<T>(c, nw, S, nsx, nsy);
+  return TbLayout<T>(nw, S, c.n_mat, nsx, nsy).bytes;
+}
+
+// Whether a scene takes the blocked step.  The second set of the E-side psi it
+// alternates with is part of a checkpoint, so the rule is kept as it was for
+// the former tile (96 columns of which 2 S + 1 were halo, psi of at most 16
+// slab rows and columns, 227 KB): states saved by either load into the other.
+template <typename T>
+bool tb2d_has_set(const xfb_handle* h) {
   const Compiled& c = h->c;
   const int S = h->tb_steps;
   if (c.dim != 2 || S <= 0 || !c.movies.empty()) return false;
-  const int TJ = kTbPitch - 1 - 2 * S;
+  constexpr int kPitch = 96, kSlab = 16;
+  const int TJ = kPitch - 1 - 2 * S;
   if (TJ < 16) return false;
-  const int ntj = (c.ny + TJ - 1) / TJ;
-  int TI = (c.nx + std::max(1, 296 / ntj) - 1) / std::max(1, 296 / ntj);
-  TI = std::min(64, std::max(16, TI));
-  // the tile's shared memory within the 227 KB a CTA may use
-  while (TI > 16 && TbLayout<T>(TI + 2 * S + 1, c.n_mat).bytes > 227u * 1024u) --TI;
-  if (TbLayout<T>(TI + 2 * S + 1, c.n_mat).bytes > 227u * 1024u) return false;
-  auto fits = [&](int n, int tile, int lo, int hi) {  // slab cells of every tile's region along one axis
+  auto bytes = [&](int ti) {
+    const size_t xi = ti + 2 * S + 1;
+    const size_t px = (3 * xi * kPitch * sizeof(T) + xi * kPitch + 15) / 16 * 16;
+    const size_t slots = px + 2ull * kSlab * kPitch * sizeof(T) + 2 * xi * kSlab * sizeof(T) + c.n_mat * 18ull * sizeof(T);
+    return (slots + (xi + kPitch) * sizeof(int) + 15) / 16 * 16 + (4ull * kPitch + 4 * xi) * sizeof(double);
+  };
+  const int per = std::max(1, 296 / ((c.ny + TJ - 1) / TJ));
+  int TI = std::min(64, std::max(16, (c.nx + per - 1) / per));
+  while (TI > 16 && bytes(TI) > kTbSmem) --TI;
+  if (bytes(TI) > kTbSmem) return false;
+  auto fits = [&](int n, int tile, int lo, int hi) {
     for (int a0 = 0; a0 < n; a0 += tile) {
       int cnt = 0;
       for (int q = std::max(0, a0 - S); q <= std::min(n - 1, a0 + tile + S); ++q) cnt += (q < lo || q >= n - hi) ? 1 : 0;
-      if (cnt > kTbSlab) return false;
+      if (cnt > kSlab) return false;
     }
     return true;
   };
-  if (!fits(c.nx, TI, c.pml[0], c.pml[1]) || !fits(c.ny, TJ, c.pml[2], c.pml[3])) return false;
-  h->tb_ti = TI;
-  h->tb_tj = TJ;
-  return true;
+  return fits(c.nx, TI, c.pml[0], c.pml[1]) && fits(c.ny, TJ, c.pml[2], c.pml[3]);
+}
+
+// Warps per CTA (tile rows) and steps per launch of the blocked 2-D step, at
+// most the caller's.  False (one launch per step) when blocking is off or the
+// scene does not take it.
+template <typename T>
+bool tb2d_plan(xfb_handle* h) {
+  const Compiled& c = h->c;
+  h->tb_warps = 0;
+  if (!tb2d_has_set<T>(h)) return false;
+  // A grid that fills the GPU with the largest tiles takes them: its launches
+  // are bound by issue slots, and the longest blocks lose more to their halo
+  // than they save.  us per step with 16 warps and S = 5 / 7 / 9 / 11: FP32
+  // 1044^2 8.2 / 6.9 / 7.1 / 7.7, 2020 x 1720 - / 12.5 / 12.2 / 11.9; FP64
+  // 1519 x 751 14.2 / 13.6 / 14.1 / -, 2020 x 1720 - / 23.9 / 24.0 / -.
+  auto tiles_of = [&](const TbGeom<T>& g) {
+    return std::ceil(static_cast<double>(c.nx) / g.ti) * std::ceil(static_cast<double>(c.ny) / g.tj);
+  };
+  const double fill = tiles_of(TbGeom<T>(kTbMaxWarps<T>, 7)) / 148.0;
+  int nw_lo = 4, S_hi = 11;
+  if (fill >= 1) {
+    nw_lo = kTbMaxWarps<T>;
+    S_hi = sizeof(T) == 4 && fill >= 3 ? 9 : 7;
+  }
+  // Smaller grids: the cheapest pair by the cost model.
+  double best = 0;
+  for (int S = h->tb_given ? h->tb_steps : S_hi; S >= 1 && !(h->tb_warps && (h->tb_given || nw_lo > 4)); S -= 2)
+    for (int nw = nw_lo; nw <= kTbMaxWarps<T>; nw += 2) {
+      const TbGeom<T> g(nw, S);
+      if (g.ti < kTbRows<T> || g.tj < kTbC) continue;
+      int nsx, nsy;
+      const size_t smem = tb2d_bytes<T>(c, nw, S, nsx, nsy);
+      if (smem > kTbSmem) continue;
+      const double tiles = tiles_of(g);
+      const int per_sm = std::max(1, std::min<int>(kTbMaxWarps<T> / nw, static_cast<int>(228u * 1024u / (smem + 1024u))));
+      // per wave, a tile's load and store and the steps of the CTAs that share an SM
+      const double cost = (kTbFixed + std::ceil(tiles / (148.0 * per_sm)) * (kTbLoad + S * per_sm * nw * kTbWarpStep<T>)) / S;
+      if (!h->tb_warps || cost < best) {
+        best = cost;
+        h->tb_warps = nw;
+        h->tb_max = S;
+      }
+    }
+  return h->tb_warps > 0;
 }
 
 // The kernel's shared-memory limit, set (and the kernel loaded) outside any
 // stream capture of the step loop.
 template <typename T>
 int tb2d_prepare(xfb_handle* h) {
-  const TbLayout<T> lay(h->tb_ti + 2 * h->tb_steps + 1, h->c.n_mat);
-  XFB_CUDA(h, cudaFuncSetAttribute(k_step2_tb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(lay.bytes)));
+  XFB_CUDA(h, cudaFuncSetAttribute(k_step2_tb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTbSmem)));
   return XFB_OK;
 }
 
@@ -55,16 +116,34 @@ int tb2d_prepare(xfb_handle* h) {
 template <typename T>
 void launch_tb2d(xfb_handle* h, int off, int S) {
   const Compiled& c = h->c;
-  const int parity = static_cast<int>((h->step + off) & 1);
-  const TbLayout<T> lay(h->tb_ti + 2 * S + 1, c.n_mat);
+  const int parity = static_cast<int>((h->step + off) & 1), nw = h->tb_warps;
+  int nsx, nsy;
+  const size_t smem = tb2d_bytes<T>(c, nw, S, nsx, nsy);
+  const TbGeom<T> g(nw, S);
   T* ez_x[2] = {as<T>(h->psi[1]), as<T>(h->psi_e1[0])};
   T* ez_y[2] = {as<T>(h->psi[2]), as<T>(h->psi_e1[1])};
   ProbeP pr{static_cast<int>(c.probes.size()), h->probe_idx, h->probe_field, h->probe_out, c.total_steps};
-  const dim3 grid((c.ny + h->tb_tj - 1) / h->tb_tj, (c.nx + h->tb_ti - 1) / h->tb_ti);
-  k_step2_tb<T><<<grid, kTbThreads, lay.bytes, h->stream>>>(
+  const dim3 grid((c.ny + g.tj - 1) / g.tj, (c.nx + g.ti - 1) / g.ti);
+  k_step2_tb<T><<<grid, 32 * nw, smem, h->stream>>>(
       grid_params<T>(h, parity), grid_params<T>(h, 1 - parity), pml_params<T>(h), psi_h_set<T>(h, parity),
       psi_h_set<T>(h, 1 - parity), ez_x[parity], ez_y[parity], ez_x[1 - parity], ez_y[1 - parity], tfsf_params(h),
-      TimeP{h->t_dev, off}, pr, S, h->tb_ti, h->tb_tj, c.n_mat, h->scratch_err);
+      TimeP{h->t_dev, off}, pr, S, c.n_mat, nsx, nsy);
+}
+
+// n steps as launches of odd step counts (each flips the sets once), as equal
+// as they can be: a launch costs the same for few steps as for many.
+template <typename T>
+void tb2d_chunk(xfb_handle* h, int n) {
+  int launches = (n + h->tb_max - 1) / h->tb_max;
+  launches += (launches ^ n) & 1;
+  int S = n / launches;
+  S -= 1 - (S & 1);
+  int longer = (n - S * launches) / 2;  // launches of S + 2 steps
+  for (int off = 0; off < n;) {
+    const int s = longer-- > 0 ? S + 2 : S;
+    launch_tb2d<T>(h, off, s);
+    off += s;
+  }
 }
 
 }  // namespace xfb
@@ -74,4 +153,5 @@ void launch_tb2d(xfb_handle* h, int off, int S) {
   template bool tb2d_plan<T>(xfb_handle*);               \
   template int tb2d_prepare<T>(xfb_handle*);             \
   template void launch_tb2d<T>(xfb_handle*, int, int);   \
+  template void tb2d_chunk<T>(xfb_handle*, int);         \
   }
