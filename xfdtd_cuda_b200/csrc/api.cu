@@ -46,9 +46,122 @@ int cuda_err(xfb_handle* h, cudaError_t e, const char* what) {
 
 
 
+namespace {
+struct PinPool {
+  std::mutex mu;
+  std::vector<void*> idle;
+  int users = 0;
+};
+// never destroyed: a handle may outlive the static objects of the process
+PinPool& pin_pool() {
+  static PinPool* pool = new PinPool;
+  return *pool;
+}
+void* pin_alloc() {
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, kPinBytes, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+void* pin_take() {
+  PinPool& pool = pin_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    if (!pool.idle.empty()) {
+      void* p = pool.idle.back();
+      pool.idle.pop_back();
+      return p;
+    }
+  }
+  return pin_alloc();
+}
+void pin_give(void* p) {
+  if (!p) return;
+  PinPool& pool = pin_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    if (pool.users > 0 && pool.idle.size() < kPinIdle) {
+      pool.idle.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+}  // namespace
+
+void pin_use(xfb_handle* h) {
+  if (h->pin_user) return;
+  h->pin_user = true;
+  PinPool& pool = pin_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  ++pool.users;
+}
+
+namespace {
+void pin_release(xfb_handle* h) {
+  if (!h->pin_user) return;
+  std::vector<void*> drop;
+  {
+    PinPool& pool = pin_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    if (--pool.users == 0) drop.swap(pool.idle);
+  }
+  for (void* p : drop) cudaFreeHost(p);
+}
+}  // namespace
+
+void pin_warm() {
+  size_t have;
+  {
+    PinPool& pool = pin_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    have = pool.idle.size();
+  }
+  for (; have < 2; ++have) pin_give(pin_alloc());
+}
+
+PinnedPair::PinnedPair() {
+  p[0] = pin_take();
+  p[1] = p[0] ? pin_take() : nullptr;
+}
+
+PinnedPair::~PinnedPair() {
+  pin_give(p[0]);
+  pin_give(p[1]);
+}
+
+namespace {
+constexpr size_t kSpareMax = 1u << 30;  // bytes of blocks kept from one init for the next
+}
+
+void free_spare(xfb_handle* h) {
+  for (auto& b : h->spare) cudaFree(b.p);
+  h->spare.clear();
+}
+
+// Ends the handle's device state.  Its cudaMalloc blocks are kept for the next
+// init (device_malloc takes those of the same size, xfb_init frees the rest),
+// up to kSpareMax bytes in all: allocating and freeing them again takes 0.8 ms
+// a block, and on a host whose driver is busy up to some 100 ms.
+void keep_blocks(xfb_handle* h) {
+  std::vector<xfb::Buf> spare;
+  size_t bytes = 0;
+  for (auto& b : h->bufs)
+    if (b.owner && bytes + b.block <= kSpareMax) {
+      bytes += b.block;
+      spare.push_back(b);
+      b.owner = false;
+    }
+  free_device(h);
+  h->spare.swap(spare);
+}
+
 void free_device(xfb_handle* h) {
   for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
   h->graphs.clear();
+  free_spare(h);
   for (auto& b : h->bufs)
     if (b.owner) cudaFree(b.p);
   h->bufs.clear();
@@ -64,11 +177,9 @@ void free_device(xfb_handle* h) {
   h->ade_runs = nullptr;
   h->n_ade_runs = -1;
   h->rb_dev = nullptr;  // one of bufs
-  for (int q = 0; q < 2; ++q) {
-    if (h->rb_host[q]) cudaFreeHost(h->rb_host[q]);
-    if (h->rb_ev[q]) cudaEventDestroy(h->rb_ev[q]);
-    h->rb_host[q] = nullptr;
-    h->rb_ev[q] = nullptr;
+  for (cudaEvent_t& ev : h->rb_ev) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
   }
   h->inited = false;
 }
@@ -82,12 +193,25 @@ constexpr size_t kAlign = 256;
 // state; not part of the checkpoint state, whose parts are listed separately).
 int device_malloc(xfb_handle* h, void** out, size_t bytes) {
   void* p = nullptr;
-  const cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return set_err(h, XFB_ERR_OOM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
+  for (auto it = h->spare.begin(); it != h->spare.end(); ++it)
+    if (it->block == bytes) {
+      p = it->p;
+      h->spare.erase(it);
+      break;
+    }
+  if (!p) {
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && !h->spare.empty()) {
+      cudaGetLastError();
+      free_spare(h);
+      e = cudaMalloc(&p, bytes);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return set_err(h, XFB_ERR_OOM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
+    }
   }
-  h->bufs.push_back({p, 0, false, true});
+  h->bufs.push_back({p, 0, false, true, bytes});
   h->bytes += bytes;
   *out = p;
   return XFB_OK;
@@ -395,6 +519,7 @@ int xfb_destroy(xfb_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_device(h);
+    pin_release(h);
     if (h->stream) cudaStreamDestroy(h->stream);
   }
   delete h;
@@ -495,10 +620,12 @@ int xfb_init(xfb_handle* h, long long total_steps) {
   }
   XFB_CUDA(h, cudaSetDevice(h->device));
   XFB_CUDA(h, cudaStreamSynchronize(h->stream));
-  free_device(h);
+  keep_blocks(h);
   size_tables(h->c, total_steps);
-  if (h->path == XFB_PATH_PLAIN && (h->c.dim != 3 || h->c.ade_kind != XFB_ADE_NONE))
+  if (h->path == XFB_PATH_PLAIN && (h->c.dim != 3 || h->c.ade_kind != XFB_ADE_NONE)) {
+    free_spare(h);
     return set_err(h, XFB_ERR_INVALID, "the plain path handles 3-D scenes without dispersive media only");
+  }
   if (h->path == XFB_PATH_AUTO) h->path = XFB_PATH_FUSED;
   int rc;
   try {
@@ -506,6 +633,7 @@ int xfb_init(xfb_handle* h, long long total_steps) {
   } catch (const std::bad_alloc&) {
     rc = set_err(h, XFB_ERR_OOM, "host allocation failed during init");
   }
+  free_spare(h);
   if (rc) {
     free_device(h);
     return rc;
@@ -1300,7 +1428,12 @@ int xfb_batch_step(xfb_batch* b, long long n) {
   if (n < 0) return batch_err(b, XFB_ERR_INVALID, "negative step count");
   if (b->step + n > b->total) return batch_err(b, XFB_ERR_RANGE, "steps beyond the count xfb_batch_init sized the run for");
   if (cudaSetDevice(b->device) != cudaSuccess) return batch_err(b, XFB_ERR_CUDA, "cudaSetDevice");
-  return b->prec == XFB_FP64 ? batch_run<double>(b, n) : batch_run<float>(b, n);
+  const int rc = b->prec == XFB_FP64 ? batch_run<double>(b, n) : batch_run<float>(b, n);
+  if (rc == XFB_OK && n > 0) {  // the read-backs' staging, pinned while the device steps
+    pin_use(b->hs[0]);
+    pin_warm();
+  }
+  return rc;
 }
 
 int xfb_batch_sync(xfb_batch* b) {

@@ -99,29 +99,20 @@ int init_device(xfb_handle* h) {
     }
   }
   // material ids in the padded layout: the dense array is copied as it is and
-  // spread into the (zeroed) padded one on the device
+  // spread into the (zeroed) padded one on the device.  It is staged in the
+  // first field, a byte a cell where that has at least four, and zeroed after.
   {
     void* p;  // same guard as the fields (the one-sweep kernel stages halo windows)
     if ((rc = alloc(h, &p, static_cast<size_t>(h->elems) + 2 * h->guard, false))) return rc;
     h->mid = static_cast<uint8_t*>(p) + h->guard;
     const size_t dense = c.mat_id.size();
-    void* tmp = nullptr;
-    if (cudaMalloc(&tmp, dense) != cudaSuccess) {
-      cudaGetLastError();
-      return set_err(h, XFB_ERR_OOM, "cudaMalloc of the material-id staging buffer failed");
-    }
-    rc = copy(h, tmp, c.mat_id.data(), dense, cudaMemcpyHostToDevice);
-    if (rc == XFB_OK) {
-      const long long rows = static_cast<long long>(nx) * ny;
-      k_spread_ids<uint8_t><<<static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 148LL * 64)), 256, 0, h->stream>>>(
-          static_cast<const uint8_t*>(tmp), h->mid, ny, nz, h->sx, h->sy, rows);
-      const cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) rc = cuda_err(h, e, "material-id spread");
-      const cudaError_t e2 = cudaStreamSynchronize(h->stream);  // before the staging buffer is freed
-      if (rc == XFB_OK && e2 != cudaSuccess) rc = cuda_err(h, e2, "material-id spread");
-    }
-    cudaFree(tmp);
-    if (rc) return rc;
+    void* tmp = h->f[XFB_EZ];
+    if ((rc = copy(h, tmp, c.mat_id.data(), dense, cudaMemcpyHostToDevice))) return rc;
+    const long long rows = static_cast<long long>(nx) * ny;
+    k_spread_ids<uint8_t><<<static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 148LL * 64)), 256, 0, h->stream>>>(
+        static_cast<const uint8_t*>(tmp), h->mid, ny, nz, h->sx, h->sy, rows);
+    XFB_CUDA(h, cudaGetLastError());
+    XFB_CUDA(h, cudaMemsetAsync(tmp, 0, dense, h->stream));
   }
   if (h->coeff_storage == XFB_COEFF_NATIVE) {
     if ((rc = upload<T>(h, &h->lut, c.coeff))) return rc;
@@ -1129,8 +1120,7 @@ void enqueue_chunk(xfb_handle* h, int n) {
   k_bump<<<1, 1, 0, h->stream>>>(h->t_dev, n);
 }
 
-template <typename T>
-bool readback_buffers(xfb_handle* h);
+inline bool readback_buffers(xfb_handle* h);
 
 template <typename T>
 int run_steps(xfb_handle* h, long long n) {
@@ -1161,7 +1151,12 @@ int run_steps(xfb_handle* h, long long n) {
   }
   // the read-back's staging buffers, allocated while the device steps (a
   // failure leaves the read-back to its unstaged form)
-  if (n > 0 && !h->rb_host[1] && !readback_buffers<T>(h)) h->err.clear();
+  if (n > 0) {
+    if (readback_buffers(h))
+      pin_warm();
+    else
+      h->err.clear();
+  }
   return XFB_OK;
 }
 
@@ -1208,36 +1203,24 @@ __global__ void k_gather_field(const T* src, T* dst, long long sx, long long sy,
   }
 }
 
-// Elements of one read-back chunk (device gather buffer and each pinned host
-// buffer hold this many elements of the compute type).
-constexpr long long kReadChunk = 4LL << 20;
-
-
-// Read-back buffers of the handle (device gather buffer, two pinned host
-// buffers, their events), allocated on first use and kept until the next
-// init or destroy.  False when any allocation fails.
-template <typename T>
-bool readback_buffers(xfb_handle* h) {
-  if (h->rb_dev && h->rb_host[0] && h->rb_host[1]) return true;
-  const size_t bytes = static_cast<size_t>(kReadChunk) * sizeof(T);
-  if (!h->rb_dev && alloc(h, &h->rb_dev, bytes, false) != XFB_OK) return false;
-  for (int q = 0; q < 2; ++q) {
-    if (!h->rb_host[q] && cudaHostAlloc(&h->rb_host[q], bytes, cudaHostAllocDefault) != cudaSuccess) {
-      h->rb_host[q] = nullptr;
+// Read-back buffers of the handle (device gather buffer, events), allocated on
+// first use and kept until the next init or destroy; the pinned host buffers
+// come from the process's pool for the length of a read.  False when any
+// allocation fails.
+inline bool readback_buffers(xfb_handle* h) {
+  pin_use(h);
+  if (!h->rb_dev && alloc(h, &h->rb_dev, kPinBytes, false) != XFB_OK) return false;
+  for (cudaEvent_t& ev : h->rb_ev)
+    if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+      ev = nullptr;
       cudaGetLastError();
       return false;
     }
-    if (!h->rb_ev[q] && cudaEventCreateWithFlags(&h->rb_ev[q], cudaEventDisableTiming) != cudaSuccess) {
-      h->rb_ev[q] = nullptr;
-      cudaGetLastError();
-      return false;
-    }
-  }
   return true;
 }
 
 // Read-back of component f into the caller's double array.  Chunks of
-// kReadChunk elements are gathered on the device in the compute type, copied
+// kPinBytes are gathered on the device in the compute type, copied
 // into pinned host buffer c & 1, and widened to double by host threads while
 // the device gathers and copies the next chunk.  The host-side gather below
 // runs when the read-back buffers cannot be allocated.
@@ -1247,7 +1230,9 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
   comp_shape(h->c, f, s);
   const long long total = static_cast<long long>(s[0]) * s[1] * s[2];
   if (total == 0) return XFB_OK;
-  if (readback_buffers<T>(h)) {
+  PinnedPair pin;
+  if (pin.ok() && readback_buffers(h)) {
+    constexpr long long kReadChunk = kPinBytes / sizeof(T);
     const T* src = static_cast<const T*>(field_ptr(h, cur_set(h), f));
     T* stage = static_cast<T*>(h->rb_dev);
     const long long nch = (total + kReadChunk - 1) / kReadChunk;
@@ -1256,7 +1241,7 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
       const unsigned blocks = static_cast<unsigned>(std::min<long long>((n + 255) / 256, 148LL * 16));
       k_gather_field<T><<<blocks, 256, 0, h->stream>>>(src, stage, h->sx, h->sy, s[1], s[2], q0, n);
       cudaError_t e = cudaGetLastError();
-      if (e == cudaSuccess) e = cudaMemcpyAsync(h->rb_host[c & 1], stage, n * sizeof(T), cudaMemcpyDeviceToHost, h->stream);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(pin.p[c & 1], stage, n * sizeof(T), cudaMemcpyDeviceToHost, h->stream);
       if (e == cudaSuccess) e = cudaEventRecord(h->rb_ev[c & 1], h->stream);
       return e;
     };
@@ -1267,7 +1252,7 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
       if (e == cudaSuccess) e = cudaEventSynchronize(h->rb_ev[c & 1]);
       if (e != cudaSuccess) break;
       const long long q0 = c * kReadChunk, n = std::min(kReadChunk, total - q0);
-      host_widen(static_cast<const T*>(h->rb_host[c & 1]), dst + q0, n);
+      host_widen(static_cast<const T*>(pin.p[c & 1]), dst + q0, n);
       h->d2h_bytes += n * static_cast<long long>(sizeof(T));
     }
     if (e != cudaSuccess) {
@@ -1293,18 +1278,19 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
 template <typename T>
 int read_bytes_t(xfb_handle* h, void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return XFB_OK;
-  if (!readback_buffers<T>(h)) {
+  PinnedPair pin;
+  if (!pin.ok() || !readback_buffers(h)) {
     h->err.clear();
     XFB_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
     XFB_CUDA(h, cudaStreamSynchronize(h->stream));
     h->d2h_bytes += static_cast<long long>(bytes);
     return XFB_OK;
   }
-  const size_t chunk = static_cast<size_t>(kReadChunk) * sizeof(T);
+  constexpr size_t chunk = kPinBytes;
   const size_t nch = (bytes + chunk - 1) / chunk;
   auto enqueue = [&](size_t c) -> cudaError_t {
     const size_t o = c * chunk, n = std::min(chunk, bytes - o);
-    cudaError_t e = cudaMemcpyAsync(h->rb_host[c & 1], static_cast<const char*>(src) + o, n, cudaMemcpyDeviceToHost,
+    cudaError_t e = cudaMemcpyAsync(pin.p[c & 1], static_cast<const char*>(src) + o, n, cudaMemcpyDeviceToHost,
                                     h->stream);
     if (e == cudaSuccess) e = cudaEventRecord(h->rb_ev[c & 1], h->stream);
     return e;
@@ -1315,7 +1301,7 @@ int read_bytes_t(xfb_handle* h, void* dst, const void* src, size_t bytes) {
     if (e == cudaSuccess) e = cudaEventSynchronize(h->rb_ev[c & 1]);
     if (e != cudaSuccess) break;
     const size_t o = c * chunk, n = std::min(chunk, bytes - o);
-    host_copy(h->rb_host[c & 1], static_cast<char*>(dst) + o, n);
+    host_copy(pin.p[c & 1], static_cast<char*>(dst) + o, n);
     h->d2h_bytes += static_cast<long long>(n);
   }
   if (e != cudaSuccess) {

@@ -19,7 +19,27 @@ struct Buf {
   size_t bytes = 0;
   bool state = false;  // part of the checkpoint state
   bool owner = true;   // p is a cudaMalloc base (freed with the handle's device state)
+  size_t block = 0;    // an owner's allocation size
 };
+
+// Pinned staging buffers of the read-backs, shared by the handles of the
+// process: a read takes two and gives them back.  Pinning costs 0.5 ms per MB,
+// so a pair per handle of 16 MB (FP32) or 32 MB (FP64) buffers cost 17 and
+// 35 ms per run, and once more 4 or 7 ms to unpin; at 4 MB a chunk's copy
+// (75 us) still hides its launches.  At most kPinIdle unused buffers are kept,
+// none once the last handle that reads back is destroyed.
+constexpr size_t kPinBytes = 4u << 20;
+constexpr size_t kPinIdle = 4;
+void pin_warm();  // have two unused buffers, as far as they can be had
+struct PinnedPair {
+  void* p[2];
+  PinnedPair();
+  ~PinnedPair();
+  PinnedPair(const PinnedPair&) = delete;
+  PinnedPair& operator=(const PinnedPair&) = delete;
+  bool ok() const { return p[0] && p[1]; }
+};
+
 
 }  // namespace xfb
 
@@ -151,13 +171,15 @@ struct xfb_handle {
   bool labc_on = false;
   void* labc_w = nullptr;
   float* labc_hist = nullptr;
-  // field read-back (read_field_t): a device gather buffer of kReadChunk
-  // elements of the compute type, two pinned host buffers of the same size
-  // (chunk c lands in buffer c & 1 while the host widens chunk c - 1 to
-  // double), their completion events; allocated by the first read-back
+  // field read-back (read_field_t): a device gather buffer of kPinBytes and
+  // the events that mark each pinned buffer's chunk as copied (chunk c lands in
+  // buffer c & 1 while the host widens chunk c - 1 to double); pin_user: the
+  // handle counts among the staging pool's users
   void* rb_dev = nullptr;
-  void* rb_host[2] = {};
   cudaEvent_t rb_ev[2] = {};
+  bool pin_user = false;
+  // cudaMalloc blocks of the previous init, offered to the next one
+  std::vector<Buf> spare;
   // bytes this handle has copied host -> device and device -> host
   long long h2d_bytes = 0, d2h_bytes = 0;
   // x-slab decomposition (xfb_set_slab): the handle updates cells
@@ -218,6 +240,9 @@ template <typename T>
 T* as(void* p) { return static_cast<T*>(p); }
 
 void free_device(xfb_handle* h);
+void keep_blocks(xfb_handle* h);
+void pin_use(xfb_handle* h);  // count the handle among the staging pool's users
+void free_spare(xfb_handle* h);
 int alloc(xfb_handle* h, void** out, size_t bytes, bool state);
 // n zeroed buffers of `bytes` each (256-byte aligned) from one cudaMalloc.
 int alloc_block(xfb_handle* h, void** out, int n, size_t bytes, bool state);
