@@ -410,17 +410,20 @@ int xfb_labc_wall_cells(const xfb_handle* h, long long* cells);
 
 /* ---- batches of scenes ---------------------------------------------------
  * No counterpart in the reference (whose SimulationHD runs one scene per
- * object).  A batch steps many 3-D scenes of one precision together: every
- * step is one launch of the one-sweep kernel over the work items of all
- * scenes, plus one launch for all TFSF auxiliary grids, replayed from CUDA
- * graphs.  Results are identical to stepping each scene alone.  The handles
+ * object).  A batch steps many 3-D scenes of one precision together, replayed
+ * from CUDA graphs.  Where every scene takes the two-pass step when stepped
+ * alone and neither the tile rows nor the launch form is set, a graph holds the
+ * scenes' steps as parallel chains.  Otherwise every step is one launch of the
+ * one-sweep kernel over the work items of all scenes, plus one launch for all
+ * TFSF line tables.  Results are identical to stepping each scene alone.  The handles
  * stay owned by the caller and are read as usual (xfb_read_field, ...) after
  * xfb_batch_sync; while in a batch they cannot be stepped, initialised or
  * destroyed on their own (XFB_ERR_STATE). */
 typedef struct xfb_batch xfb_batch;
 /* Group n created handles (same precision, 3-D, one device). */
 int xfb_batch_create(xfb_handle* const* handles, int n, xfb_batch** out);
-/* Tile rows of the one-sweep kernel: 0 = autotune on the first steps (default), 8, 14 or 16. */
+/* Tile rows of the one-sweep kernel: 0 = autotune on the first steps (default),
+ * 8, 14 or 16, which take a batch off the two-pass step. */
 int xfb_batch_set_tile(xfb_batch* b, int rows);
 /* How the steps are launched.  XFB_BATCH_PER_STEP: one launch of the
  * one-sweep kernel per step.  XFB_BATCH_PERSISTENT: one launch per chunk of
@@ -431,20 +434,22 @@ int xfb_batch_set_tile(xfb_batch* b, int rows);
  * step of the others.  Only for batches whose scenes record no monitors (NF2FF,
  * probes, movies) and run no separate ADE pass, which the per-step form
  * launches between steps; otherwise XFB_ERR_INVALID.  XFB_BATCH_AUTO (default)
- * times both on the first steps, together with the tile rows, and keeps the
- * faster. */
+ * takes the two-pass step where it can (reported as XFB_BATCH_PER_STEP), else
+ * times both forms on the first steps, together with the tile rows, and keeps
+ * the faster. */
 enum xfb_batch_launch { XFB_BATCH_AUTO = 0, XFB_BATCH_PER_STEP = 1, XFB_BATCH_PERSISTENT = 2 };
 int xfb_batch_set_launch(xfb_batch* b, int launch);
 /* The launch form in use (0 before the first step). */
 int xfb_batch_launch_form(const xfb_batch* b, int* launch);
-/* xfb_init every scene for total_steps steps (one-sweep path) and build the batch's work list. */
+/* xfb_init every scene for total_steps steps and build the batch's work list. */
 int xfb_batch_init(xfb_batch* b, long long total_steps);
 /* Advance every scene n steps (asynchronous). */
 int xfb_batch_step(xfb_batch* b, long long n);
 /* XFB_ERR_TIMEOUT as for xfb_sync when a bounded wait of the step ran out. */
 int xfb_batch_sync(xfb_batch* b);
-/* Poll limit of the batch step's bounded waits (after xfb_batch_init), as
- * xfb_set_wait_limit. */
+/* Poll limit of the one-sweep batch step's bounded waits (after
+ * xfb_batch_init), as xfb_set_wait_limit; takes a batch off the two-pass step,
+ * which has none. */
 int xfb_batch_set_wait_limit(xfb_batch* b, int polls);
 /* n steps between CUDA events on the batch's stream; *ms = device time. */
 int xfb_batch_timed_step(xfb_batch* b, long long n, double* ms);

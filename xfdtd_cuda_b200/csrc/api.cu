@@ -1348,10 +1348,47 @@ int xfb_batch_create(xfb_handle* const* handles, int n, xfb_batch** out) {
   return XFB_OK;
 }
 
+// Which step the scenes take: the two-pass one in chains, else (and for all of
+// them) the batch's one-sweep kernels, which alternate the field sets.
+static int batch_plan(xfb_batch* b) {
+  b->two_pass = b->prec == XFB_FP64 ? tp_batch_plan<double>(b) : tp_batch_plan<float>(b);
+  if (!b->two_pass)
+    for (xfb_handle* h : b->hs) h->two_pass = false;
+  const size_t n = b->two_pass ? std::min<size_t>(b->hs.size(), kBatchChains) : 0;
+  while (b->chains.size() < n) {
+    cudaStream_t s;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
+      return batch_err(b, XFB_ERR_CUDA, "cudaStreamCreate");
+    b->chains.push_back(s);
+  }
+  while (n && b->chain_ev.size() < n + 1) {
+    cudaEvent_t ev;
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+      return batch_err(b, XFB_ERR_CUDA, "cudaEventCreate");
+    b->chain_ev.push_back(ev);
+  }
+  return XFB_OK;
+}
+
+// The caller chose a form of the one-sweep step: the scenes' state moves to
+// the set it reads.
+static int batch_leave(xfb_batch* b) {
+  if (!b->two_pass) return XFB_OK;
+  cudaSetDevice(b->device);
+  for (xfb_handle* h : b->hs)
+    if (int rc = tp_leave(h)) return batch_err(b, rc, h->err);
+  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
+  b->graphs.clear();
+  b->two_pass = false;
+  return XFB_OK;
+}
+
 int xfb_batch_set_tile(xfb_batch* b, int rows) {
   if (!b) return set_err(nullptr, XFB_ERR_INVALID, "null batch");
   if (rows != 0 && rows != 8 && rows != 14 && rows != 16)
     return batch_err(b, XFB_ERR_INVALID, "tile rows must be 0 (autotune), 8, 14 or 16");
+  if (rows != 0)
+    if (int rc = batch_leave(b)) return rc;
   b->tile_req = rows;
   b->tile = -1;
   return XFB_OK;
@@ -1363,6 +1400,8 @@ int xfb_batch_set_launch(xfb_batch* b, int launch) {
     return batch_err(b, XFB_ERR_INVALID, "launch form must be XFB_BATCH_AUTO, XFB_BATCH_PER_STEP or XFB_BATCH_PERSISTENT");
   if (b->inited && launch == XFB_BATCH_PERSISTENT && !b->persist_ok)
     return batch_err(b, XFB_ERR_INVALID, "persistent batch launches need scenes without monitors or a separate ADE pass");
+  if (launch != XFB_BATCH_AUTO)
+    if (int rc = batch_leave(b)) return rc;
   b->launch_req = launch;
   b->launch = -1;
   b->tile = -1;
@@ -1401,13 +1440,13 @@ int xfb_batch_init(xfb_batch* b, long long total_steps) {
     int rc = xfb_init(h, total_steps);
     h->batch = b;
     if (rc) return batch_err(b, rc, "scene init failed: " + h->err);
-    h->two_pass = false;  // the batch's kernels alternate the field sets
     b->cells += static_cast<long long>(h->c.nx) * h->c.ny * h->c.nz;
   }
   if (cudaSetDevice(dev) != cudaSuccess) return batch_err(b, XFB_ERR_CUDA, "cudaSetDevice");
   if (!b->stream && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     return batch_err(b, XFB_ERR_CUDA, "cudaStreamCreate");
   int rc;
+  if ((rc = batch_plan(b))) return rc;
   try {
     rc = b->prec == XFB_FP64 ? batch_init<double>(b) : batch_init<float>(b);
   } catch (const std::bad_alloc&) {
@@ -1459,6 +1498,7 @@ int xfb_batch_set_wait_limit(xfb_batch* b, int polls) {
   if (!b) return set_err(nullptr, XFB_ERR_INVALID, "null batch");
   if (!b->inited) return batch_err(b, XFB_ERR_STATE, "batch not initialised");
   if (polls < 0) return batch_err(b, XFB_ERR_INVALID, "negative poll limit");
+  if (int rc = batch_leave(b)) return rc;  // the two-pass step has no waits
   cudaSetDevice(b->device);
   cudaError_t e = cudaMemcpyAsync(b->err_dev + 1, &polls, sizeof(int), cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -1510,6 +1550,8 @@ int xfb_batch_destroy(xfb_batch* b) {
     }
   }
   batch_free(b);
+  for (cudaStream_t s : b->chains) cudaStreamDestroy(s);
+  for (cudaEvent_t ev : b->chain_ev) cudaEventDestroy(ev);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return XFB_OK;

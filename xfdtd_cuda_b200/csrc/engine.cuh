@@ -1518,10 +1518,45 @@ void batch_enqueue_step(xfb_batch* b, int off, int t) {
   }
 }
 
+// n two-pass steps of every scene.  A scene's steps depend on nothing of
+// another scene, so a graph holds them as parallel chains and one scene's
+// launches fill the SMs that another's last wave leaves idle.  At most
+// kBatchChains chains, scenes handed out largest first to the shortest chain.
+template <typename T>
+void batch_chains(xfb_batch* b, int n) {
+  const int nch = static_cast<int>(b->chains.size());
+  std::vector<std::vector<xfb_handle*>> of(nch);
+  std::vector<long long> load(nch, 0);
+  auto cells = [](const xfb_handle* h) { return static_cast<long long>(h->c.nx) * h->c.ny * h->c.nz; };
+  std::vector<xfb_handle*> hs = b->hs;
+  std::stable_sort(hs.begin(), hs.end(), [&](const xfb_handle* a, const xfb_handle* c) { return cells(a) > cells(c); });
+  for (xfb_handle* h : hs) {
+    const int q = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
+    of[q].push_back(h);
+    load[q] += cells(h);
+  }
+  cudaEventRecord(b->chain_ev[nch], b->stream);
+  for (int q = 0; q < nch; ++q) {
+    cudaStreamWaitEvent(b->chains[q], b->chain_ev[nch], 0);
+    for (int off = 0; off < n; ++off)
+      for (xfb_handle* h : of[q]) {
+        const TimeP tp{b->t_dev, off};
+        const Compiled& c = h->c;
+        tp_update<T>(h, tp, b->chains[q], nullptr);
+        if (c.nf_on || c.td_on || !c.probes.empty() || !c.movies.empty())
+          enqueue_records<T>(h, static_cast<int>((b->step + off) & 1), tp, b->chains[q], nullptr);
+      }
+    cudaEventRecord(b->chain_ev[q], b->chains[q]);
+    cudaStreamWaitEvent(b->stream, b->chain_ev[q], 0);
+  }
+}
+
 template <typename T>
 int batch_chunk(xfb_batch* b, int n, int t, bool graph, int launch) {
   auto enqueue = [&]() {
-    if (launch == XFB_BATCH_PERSISTENT) {
+    if (b->two_pass) {
+      batch_chains<T>(b, n);
+    } else if (launch == XFB_BATCH_PERSISTENT) {
       if (b->n_items[t]) {
         TimeP tp{b->t_dev, 0};
         const int parity = static_cast<int>(b->step & 1);
@@ -1536,7 +1571,8 @@ int batch_chunk(xfb_batch* b, int n, int t, bool graph, int launch) {
   };
   cudaError_t e = cudaSuccess;
   if (graph) {
-    const int key = ((n * 2 + static_cast<int>(b->step & 1)) * 3 + launch) * kStepTileCount + t;
+    // (the two-pass step's sets stay: one graph per length)
+    const int key = b->two_pass ? -n : ((n * 2 + static_cast<int>(b->step & 1)) * 3 + launch) * kStepTileCount + t;
     auto it = b->graphs.find(key);
     if (it == b->graphs.end()) {
       cudaGraph_t g;
@@ -1623,6 +1659,18 @@ inline void tile_cache_put(const std::string& key, int tile) {
 template <typename T>
 int batch_run(xfb_batch* b, long long n) {
   int rc;
+  if (b->two_pass) {
+    b->tile = 1;
+    b->launch = XFB_BATCH_PER_STEP;
+    // a chunk's graph of at most some 2000 launches
+    const long long most = std::max<long long>(4, std::min<long long>(b->graph_steps, 1024 / static_cast<long long>(b->hs.size())));
+    while (n > 0) {
+      const int chunk = static_cast<int>(std::min(n, most));
+      if ((rc = batch_chunk<T>(b, chunk, b->tile, true, b->launch))) return rc;
+      n -= chunk;
+    }
+    return XFB_OK;
+  }
   // candidate launch forms: per step always, persistent when the scenes allow
   std::vector<int> forms;
   if (b->launch_req != XFB_BATCH_PERSISTENT) forms.push_back(XFB_BATCH_PER_STEP);

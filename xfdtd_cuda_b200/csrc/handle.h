@@ -194,6 +194,8 @@ struct xfb_handle {
 // step over the work items of every scene, or one persistent launch for a
 // chunk of steps (k_step3_persist).  The handles stay owned by the caller;
 // the batch owns only its tables, stream, counters and graphs.
+constexpr int kBatchChains = 16;  // parallel chains of a batch's two-pass step, at most
+
 struct xfb_batch {
   std::vector<xfb_handle*> hs;
   std::string err;
@@ -222,6 +224,11 @@ struct xfb_batch {
   void* pscene_items[3] = {};
   unsigned* queue = nullptr;
   long long lines_work = 0;  // TFSF line entries of the largest scene (0: no scene has a TFSF source)
+  // two-pass step of every scene (batch_chains): a captured stream per chain
+  // of scenes, the fork and the chains' join events
+  bool two_pass = false;
+  std::vector<cudaStream_t> chains;
+  std::vector<cudaEvent_t> chain_ev;
 };
 
 namespace xfb {
@@ -301,6 +308,7 @@ template <typename T> void launch_nonfinite(xfb_handle* h);
 // two-pass 3-D step (twopass_f32.cu, twopass_f64.cu)
 template <typename T> bool tp_plan(const xfb_handle* h);
 template <typename T> int tp_normalise(xfb_handle* h);
+template <typename T> bool tp_batch_plan(const xfb_batch* b);
 // Back to the one-sweep kernels from the current state (monitor reads, state
 // and results are unaffected).
 int tp_leave(xfb_handle* h);

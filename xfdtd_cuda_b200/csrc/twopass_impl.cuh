@@ -45,6 +45,22 @@ bool tp_plan(const xfb_handle* h) {
   return false;
 }
 
+// Whether a batch left to the library takes the two-pass step for its scenes.
+// All of them must (and in FP32 round alike whichever tile the one-sweep
+// autotune would have picked).  Before and after, us per step: FP32 4 scenes of
+// 48..64 cells a side 129 -> 30, 16 of 60..120 950 -> 447, 64 of 64..256 11870
+// -> 8215 (4.9 TB/s); FP64 16 of 24..40 344 -> 100, 16 of 60..120 1618 -> 781.
+template <typename T>
+bool tp_batch_plan(const xfb_batch* b) {
+  if (b->tile_req != 0 || b->launch_req != XFB_BATCH_AUTO) return false;
+  for (const xfb_handle* h : b->hs) {
+    if (!h->two_pass) return false;
+    for (int t = 0; sizeof(T) == 4 && t < kStepTileCount; ++t)
+      if (tp_mixed_rounding(h, kStepTileRows[t])) return false;
+  }
+  return true;
+}
+
 template <typename T>
 TpCols tp_columns(const Compiled& c) {
   constexpr int V = Vec<T>::V;
@@ -151,6 +167,10 @@ int tp_normalise(xfb_handle* h) {
   }
   XFB_CUDA(h, cudaStreamSynchronize(s));
   h->live = want;
+  if (h->batch) {  // its step graphs name the set
+    for (auto& kv : h->batch->graphs) cudaGraphExecDestroy(kv.second);
+    h->batch->graphs.clear();
+  }
   return XFB_OK;
 }
 
@@ -161,4 +181,5 @@ int tp_normalise(xfb_handle* h) {
   template bool tp_plan<T>(const xfb_handle*);                                      \
   template void tp_update<T>(xfb_handle*, TimeP, cudaStream_t, Prof*);              \
   template int tp_normalise<T>(xfb_handle*);                                        \
+  template bool tp_batch_plan<T>(const xfb_batch*);                                 \
   }

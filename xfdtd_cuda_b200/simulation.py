@@ -847,10 +847,12 @@ class Handle:
 
 
 class Batch:
-    """Steps many 3-D scenes of one precision together (xfb_batch_*): one
-    launch of the one-sweep kernel per step over the work items of every
-    scene, or one persistent launch per chunk of steps (``launch``:
-    L.BATCH_AUTO picks the faster on the first steps).  The Handles stay
+    """Steps many 3-D scenes of one precision together (xfb_batch_*): the
+    scenes' two-pass steps as parallel chains of a graph where every scene
+    takes them; else, or with ``tile_rows`` or ``launch`` set, one launch of
+    the one-sweep kernel per step over the work items of every scene, or one
+    persistent launch per chunk of steps (L.BATCH_AUTO picks the faster on the
+    first steps).  The Handles stay
     usable for read-back after ``sync()``."""
 
     def __init__(self, handles, tile_rows: int = 0, launch: int = L.BATCH_AUTO):
