@@ -176,6 +176,7 @@ void free_device(xfb_handle* h) {
   h->step_err = nullptr;
   h->ade_runs = nullptr;
   h->n_ade_runs = -1;
+  h->ade_planes = nullptr;
   h->rb_dev = nullptr;  // one of bufs
   for (cudaEvent_t& ev : h->rb_ev) {
     if (ev) cudaEventDestroy(ev);
@@ -306,7 +307,7 @@ int launches_per_step(const xfb_handle* h) {
   }
   int bulk = 2;  // H and E half-steps
   if (h->two_pass) {
-    bulk += h->ade_deferred && h->n_ade_runs > 0 ? 1 : 0;  // k_tp_ade
+    bulk += h->ade_deferred && h->n_ade_runs > 0 && !tp_ade_inside(h) ? 1 : 0;  // k_tp_ade
   } else if (fused(h)) {
     bulk = c.dim == 2 ? 1
                       : (h->n_step_items[step_tile_index(h->tj)] > 0 ? 1 : 0) + (h->ade_deferred ? 1 : 0) +

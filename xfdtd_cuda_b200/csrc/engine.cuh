@@ -795,7 +795,15 @@ inline int upload_ade_runs(xfb_handle* h) {
   if (runs.empty()) return XFB_OK;
   int rc = alloc(h, &h->ade_runs, runs.size() * sizeof(int2), false);
   if (rc) return rc;
-  return copy(h, h->ade_runs, runs.data(), runs.size() * sizeof(int2), cudaMemcpyHostToDevice);
+  if ((rc = copy(h, h->ade_runs, runs.data(), runs.size() * sizeof(int2), cudaMemcpyHostToDevice))) return rc;
+  std::vector<int> first(h->c.nx + 1, 0);  // runs are in plane order
+  for (const int2& r : runs) ++first[(r.x & 0xffff) + 1];
+  h->ade_plane_max = *std::max_element(first.begin(), first.end());
+  for (int i = 0; i < h->c.nx; ++i) first[i + 1] += first[i];
+  h->ade_plane[0] = runs.front().x & 0xffff;
+  h->ade_plane[1] = (runs.back().x & 0xffff) + 1;
+  if ((rc = alloc(h, &h->ade_planes, first.size() * sizeof(int), false))) return rc;
+  return copy(h, h->ade_planes, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice);
 }
 
 // The deferred ADE pass of one step (E^n in field set `parity`, the plain

@@ -164,6 +164,10 @@ struct xfb_handle {
   // its work list: runs of dispersive cells (k_ade_runs); -1: no list (k_ade_box)
   void* ade_runs = nullptr;
   int n_ade_runs = -1;
+  // the two-pass step's view of it: the first run of every plane (int[nx + 1]),
+  // the planes that have runs, and the most runs of one plane
+  void* ade_planes = nullptr;
+  int ade_plane[2] = {}, ade_plane_max = 0;
   // set while a batch steps this handle (xfb_batch_*)
   xfb_batch* batch = nullptr;
   // learned absorbing boundary (xfb_set_learned_abc): BF16 weights and the
@@ -306,6 +310,17 @@ template <typename T> int read_bytes_t(xfb_handle* h, void* dst, const void* src
 template <typename T> int write_field_t(xfb_handle* h, int f, const double* src);
 template <typename T> void launch_nonfinite(xfb_handle* h);
 // two-pass 3-D step (twopass_f32.cu, twopass_f64.cu)
+// Whether the two-pass step's E pass takes the dispersive cells in blocks of
+// its own instead of leaving them to k_tp_ade: up to kTpAdePoles poles (more
+// spill in its registers), and fields of at most 600 MB: where the 126 MB L2
+// holds a good part of them the overlap pays.  us per step apart and inside:
+// 128x152x136 Debye FP64 (153 MB) 105 and 97; Drude-Lorentz FP32 284^3 (600 MB)
+// 520 and 515, 408^3 (1.7 GB) 1188 and 1204, where DRAM serves one access
+// pattern better than two at once.
+constexpr int kTpAdePoles = 2;
+inline bool tp_ade_inside(const xfb_handle* h) {
+  return h->c.ade_poles <= kTpAdePoles && 6.0 * h->elems * h->esize <= 600e6;
+}
 template <typename T> bool tp_plan(const xfb_handle* h);
 template <typename T> int tp_normalise(xfb_handle* h);
 template <typename T> bool tp_batch_plan(const xfb_batch* b);

@@ -338,10 +338,9 @@ __device__ __forceinline__ T ade_e(const AdeP<T>& a, int comp, long long bi, int
 // reference applies after the ADE update.
 // ADE update of one dispersive cell of the box: E^n in `ec`, the plain eNext
 // values in `pl`, E^{n+1} to `d`.
-template <typename T>
+template <typename T, int MP = 4>  // MP: XFB_MAX_POLES, or fewer where ad.P is known to be at most that
 __device__ __forceinline__ void ade_cell(const GridP<T>& d, const AdeP<T>& ad, int i, int j, int k, long long idx,
                                          int m, const T (&ec)[3], const T (&pl)[3]) {
-  constexpr int MP = 4;  // XFB_MAX_POLES
   const long long bi = static_cast<long long>(i - ad.b0) * ad.bsx + static_cast<long long>(j - ad.b2) * ad.bsy + (k - ad.b4);
   const bool upd[3] = {j > 0 && k > 0, i > 0 && k > 0, i > 0 && j > 0};
   T* dd[3] = {d.ex, d.ey, d.ez};

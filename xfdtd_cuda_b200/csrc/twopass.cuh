@@ -15,8 +15,9 @@
 // In-place order: H^{n+1/2} of a cell needs its own old H and E^n of its upper
 // neighbours, so the H pass writes only H and reads only E; E^{n+1} likewise
 // writes only E and reads only H.  The polarisation currents of dispersive
-// cells are advanced by k_tp_ade, which updates E of those cells entirely
-// (the E pass leaves them as E^n), one warp per run of cells; when a
+// cells are advanced by blocks of the E pass or by k_tp_ade, which update E of
+// those cells entirely (the pass's vectors leave them as E^n), one warp per run
+// of cells; when a
 // dispersive cell also takes a TFSF or CPML correction the E pass does the
 // recursion itself.  The arithmetic and its order are those of k_h3 / k_e3 and
 // of the one-sweep bodies: FP64 results are bit-identical, FP32 results equal
@@ -24,7 +25,7 @@
 //
 // What bounds it, measured on a B200 (us per step, with NF2FF and probes; the
 // one-sweep step before): 156^3 FP32 69 (149), FP64 122 (240); 80x72x88 FP32 21
-// (66); 36x32x40 FP64 17 (81); 128x152x136 Debye FP64 105 (244); 408^3
+// (66); 36x32x40 FP64 17 (81); 128x152x136 Debye FP64 97 (244); 408^3
 // Drude-Lorentz FP32 1190 (1356).  At 408^3 the H pass moves 2.9 GB in 0.45 ms,
 // 85 % of the copy bandwidth with what L2 keeps; at 156^3 load latency
 // dominates (20 warps per SM, 4 TB/s of DRAM and 44 % L2 hits); below 0.5 M
@@ -77,7 +78,15 @@ struct TpArgs {
   AdeP<T> ad;      // kind kAdeNone unless the E pass does the recursion itself
   const T* lut8;   // [n_mat][8]
   int zvec;        // z-slab psi rows hold whole aligned vectors
-  unsigned disp[8];  // materials whose cells k_tp_ade updates (bit per id)
+  unsigned disp[8];  // materials of the dispersive cells outside the E pass's vectors (bit per id)
+  // those cells' runs, the first run of each plane, the planes that have any,
+  // and the blocks of a plane: its vectors' and (E pass with runs) its runs'
+  AdeP<T> ar;
+  GridP<T> g;
+  const int2* runs;
+  const int* run_first;
+  int run_lo, run_hi;
+  unsigned nblk, nade;
 };
 
 template <typename T>
@@ -85,22 +94,22 @@ __device__ __forceinline__ T& tp_at(const TpArgs<T>& a, int f, unsigned off) {
   return *reinterpret_cast<T*>(a.f[f] + off);
 }
 
-// Row and column of this thread's vector (false: none); i: the plane the CTA
-// takes.  The H pass walks the planes up and the E pass down, so each pass
+// Row and column of this thread's vector (false: none); bx: the CTA's block
+// among its plane's.  The H pass walks the planes up and the E pass down, so each pass
 // starts on the planes the last one left in L2.
 template <typename T>
-__device__ __forceinline__ bool tp_cell(const TpArgs<T>& a, int& j, int& k0) {
+__device__ __forceinline__ bool tp_cell(const TpArgs<T>& a, unsigned bx, int& j, int& k0) {
   const TpCols& c = a.c;
   int q;
-  if (blockIdx.x < c.bp) {
-    const unsigned t = blockIdx.x * kTpThreads + threadIdx.x;
+  if (bx < c.bp) {
+    const unsigned t = bx * kTpThreads + threadIdx.x;
     if (t >= static_cast<unsigned>(a.ny) * static_cast<unsigned>(c.np)) return false;
     j = static_cast<int>(c.np > 1 ? __umulhi(t, c.mp) : t);
     q = c.lo + static_cast<int>(t) - j * c.np;
     if (q >= c.c1) q += c.n1;
     if (q >= c.c2) q += c.n2;
   } else {
-    const unsigned t = (blockIdx.x - c.bp) * kTpThreads + threadIdx.x;
+    const unsigned t = (bx - c.bp) * kTpThreads + threadIdx.x;
     if (t >= static_cast<unsigned>(a.ny) * static_cast<unsigned>(c.ns)) return false;
     j = static_cast<int>(c.ns > 1 ? __umulhi(t, c.ms) : t);
     q = static_cast<int>(t) - j * c.ns;
@@ -273,7 +282,7 @@ __device__ __noinline__ void tp_e_cells(const TpArgs<T>& a, int i, int j, int k0
   for (int k = k0; k < min(k0 + Vec<T>::V, a.nz); ++k) {
     const unsigned o = tp_off(a, i, j, k), ox = o - a.sxb, oy = o - a.syb, oz = o - sizeof(T);
     const int m = a.mid[o / sizeof(T)];
-    if ((a.disp[m >> 5] >> (m & 31)) & 1u) continue;  // k_tp_ade's cell
+    if ((a.disp[m >> 5] >> (m & 31)) & 1u) continue;  // a run's cell
     const bool upd_x = j > 0 && k > 0, upd_y = i > 0 && k > 0, upd_z = i > 0 && j > 0;
     const C4<T> cf = ld_c4(a.lut8 + 8 * m);
     const T hx = tp_at(a, 3, o), hy = tp_at(a, 4, o), hz = tp_at(a, 5, o);
@@ -321,7 +330,7 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_h(const __grid_con
   constexpr int V = Vec<T>::V;
   const int i = blockIdx.y;
   int j, k0;
-  if (!tp_cell(a, j, k0)) return;
+  if (!tp_cell(a, blockIdx.x, j, k0)) return;
   const unsigned o = tp_off(a, i, j, k0), ox = o + a.sxb, oy = o + a.syb;
   Vec<T> ex, ey, ez, eyn, ezn, exj, ezj, hx, hy, hz;
   ex.ld(a.f[0] + o); ey.ld(a.f[1] + o); ez.ld(a.f[2] + o);
@@ -424,12 +433,66 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_h(const __grid_con
   hx.st(a.f[3] + o); hy.st(a.f[4] + o); hz.st(a.f[5] + o);
 }
 
+// E update of the dispersive cells of a run (E pass of the other cells leaves
+// them, and they read only H and their own E): the plain eNext value from
+// H^{n+1/2} and the ADE recursion of ade_box_cell on it, one warp per run of
+// at most 32 cells inside a 32-aligned k segment (the runs of k_ade_runs).
+template <typename T, int MP>
+__device__ __forceinline__ void tp_ade_run(const TpArgs<T>& a, int q) {
+  const int lane = threadIdx.x & 31;
+  const int2 r = a.runs[q];
+  const int lo = (r.y >> 16) & 0xff, hi = static_cast<int>(static_cast<unsigned>(r.y) >> 24);
+  if (lane < lo || lane >= hi) return;
+  const int i = r.x & 0xffff, j = static_cast<int>(static_cast<unsigned>(r.x) >> 16), k = (r.y & 0xffff) + lane;
+  const unsigned o = tp_off(a, i, j, k), ox = o - a.sxb, oy = o - a.syb, oz = o - sizeof(T);
+  const int m = a.mid[o / sizeof(T)];
+  const T hx = tp_at(a, 3, o), hy = tp_at(a, 4, o), hz = tp_at(a, 5, o);
+  const T hx_km = tp_at(a, 3, oz), hy_km = tp_at(a, 4, oz), hx_jm = tp_at(a, 3, oy), hz_jm = tp_at(a, 5, oy);
+  const T hy_p = tp_at(a, 4, ox), hz_p = tp_at(a, 5, ox);
+  const T ec[3] = {tp_at(a, 0, o), tp_at(a, 1, o), tp_at(a, 2, o)};
+  const C4<T> cf = ld_c4(a.lut8 + 8 * m);
+  T pl[3];
+  pl[0] = e_next(cf.c, ec[0], cf.z, hy - hy_km, cf.y, hz - hz_jm);
+  pl[1] = e_next(cf.c, ec[1], cf.x, hz - hz_p, cf.z, hx - hx_km);
+  pl[2] = e_next(cf.c, ec[2], cf.y, hx - hx_jm, cf.x, hy - hy_p);
+  ade_cell<T, MP>(a.g, a.ar, i, j, k, i * a.g.sx + j * a.g.sy + k, m, ec, pl);
+}
+
+// All runs, a pass of its own where tp_ade_inside says so.
 template <typename T>
+__global__ void __launch_bounds__(128) k_tp_ade(const __grid_constant__ TpArgs<T> a, int n_runs) {
+  const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (q < n_runs) tp_ade_run<T, 4>(a, q);
+}
+
+// kRuns: the grid is one row of blocks, and every plane that has dispersive
+// runs has nade blocks for them (a warp per run) after its vectors' blocks.
+// Beside the vectors of their plane the runs find the H that these read in L2,
+// and the two kinds of loads overlap (tp_ade_inside).
+template <typename T, bool kRuns>
 __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_e(const __grid_constant__ TpArgs<T> a) {
   constexpr int V = Vec<T>::V;
-  const int i = a.nx - 1 - static_cast<int>(blockIdx.y);
+  int y = static_cast<int>(blockIdx.y);
+  unsigned bx = blockIdx.x;
+  if constexpr (kRuns) {
+    const unsigned top = (a.nx - a.run_hi) * a.nblk, mid = (a.run_hi - a.run_lo) * (a.nblk + a.nade);
+    unsigned per = a.nblk;
+    if (bx >= top + mid) { y = a.nx - a.run_lo; bx -= top + mid; }
+    else if (bx >= top) { y = a.nx - a.run_hi; bx -= top; per += a.nade; }
+    const unsigned q = bx / per;
+    y += static_cast<int>(q);
+    bx -= q * per;
+  }
+  const int i = a.nx - 1 - y;
+  if constexpr (kRuns) {
+    if (bx >= a.nblk) {
+      const int q = a.run_first[i] + static_cast<int>((bx - a.nblk) * (kTpThreads / 32) + (threadIdx.x >> 5));
+      if (q < a.run_first[i + 1]) tp_ade_run<T, kTpAdePoles>(a, q);
+      return;
+    }
+  }
   int j, k0;
-  if (!tp_cell(a, j, k0)) return;
+  if (!tp_cell(a, bx, j, k0)) return;
   const unsigned o = tp_off(a, i, j, k0), ox = o - a.sxb, oy = o - a.syb;
   Vec<T> hx, hy, hz, hxj, hzj, hyi, hzi, ex, ey, ez;
   hx.ld(a.f[3] + o); hy.ld(a.f[4] + o); hz.ld(a.f[5] + o);
@@ -448,7 +511,7 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_e(const __grid_con
   const int sxp = slab(i, a.nx, pm.L[0], pm.L[1]);
   const int syp = slab(j, a.ny, pm.L[2], pm.L[3]);
   const bool zsl = k0 < pm.L[4] || k0 + V > a.nz - pm.L[5];
-  // cells to leave as they are: dispersive ones, which k_tp_ade updates
+  // cells to leave as they are: dispersive ones of the runs
   unsigned keep = 0;
   bool inline_ade = false;
 #pragma unroll
@@ -545,7 +608,7 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_e(const __grid_con
         ex.a[v] = tp_at(a, 0, ov); ey.a[v] = tp_at(a, 1, ov); ez.a[v] = tp_at(a, 2, ov);
       }
   }
-  if (keep) {  // the vector also holds cells of k_tp_ade
+  if (keep) {  // the vector also holds cells of runs
 #pragma unroll
     for (int v = 0; v < V; ++v)
       if (!((keep >> v) & 1u)) {
@@ -555,34 +618,6 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_e(const __grid_con
     return;
   }
   ex.st(a.f[0] + o); ey.st(a.f[1] + o); ez.st(a.f[2] + o);
-}
-
-// E update of the dispersive cells of a two-pass step (before or after the E
-// pass, which does not touch them): the plain eNext value from H^{n+1/2} and
-// the ADE recursion of ade_box_cell on it, one warp per run of at most 32
-// cells inside a 32-aligned k segment (the runs of k_ade_runs).
-template <typename T>
-__global__ void __launch_bounds__(128) k_tp_ade(const __grid_constant__ TpArgs<T> a, const __grid_constant__ GridP<T> g,
-                                                const __grid_constant__ AdeP<T> ad, const int2* runs, int n_runs) {
-  const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (q >= n_runs) return;
-  const int lane = threadIdx.x & 31;
-  const int2 r = runs[q];
-  const int lo = (r.y >> 16) & 0xff, hi = static_cast<int>(static_cast<unsigned>(r.y) >> 24);
-  if (lane < lo || lane >= hi) return;
-  const int i = r.x & 0xffff, j = static_cast<int>(static_cast<unsigned>(r.x) >> 16), k = (r.y & 0xffff) + lane;
-  const unsigned o = tp_off(a, i, j, k), ox = o - a.sxb, oy = o - a.syb, oz = o - sizeof(T);
-  const int m = a.mid[o / sizeof(T)];
-  const T hx = tp_at(a, 3, o), hy = tp_at(a, 4, o), hz = tp_at(a, 5, o);
-  const T hx_km = tp_at(a, 3, oz), hy_km = tp_at(a, 4, oz), hx_jm = tp_at(a, 3, oy), hz_jm = tp_at(a, 5, oy);
-  const T hy_p = tp_at(a, 4, ox), hz_p = tp_at(a, 5, ox);
-  const T ec[3] = {tp_at(a, 0, o), tp_at(a, 1, o), tp_at(a, 2, o)};
-  const C4<T> cf = ld_c4(a.lut8 + 8 * m);
-  T pl[3];
-  pl[0] = e_next(cf.c, ec[0], cf.z, hy - hy_km, cf.y, hz - hz_jm);
-  pl[1] = e_next(cf.c, ec[1], cf.x, hz - hz_p, cf.z, hx - hx_km);
-  pl[2] = e_next(cf.c, ec[2], cf.y, hx - hx_jm, cf.x, hy - hy_p);
-  ade_cell(g, ad, i, j, k, i * g.sx + j * g.sy + k, m, ec, pl);
 }
 
 }  // namespace xfb

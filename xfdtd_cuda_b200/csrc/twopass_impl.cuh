@@ -129,6 +129,14 @@ TpArgs<T> tp_args(xfb_handle* h, TimeP tp) {
     for (size_t m = 0; m < c.mat_disp.size(); ++m)
       if (c.mat_disp[m]) a.disp[m >> 5] |= 1u << (m & 31);
   }
+  a.ar = ade_params<T>(h);
+  a.g = grid_params<T>(h, h->live);
+  a.runs = static_cast<const int2*>(h->ade_runs);
+  a.run_first = static_cast<const int*>(h->ade_planes);
+  a.run_lo = h->ade_plane[0];
+  a.run_hi = h->ade_plane[1];
+  a.nblk = a.c.bp + (c.ny * a.c.ns + kTpThreads - 1) / kTpThreads;
+  a.nade = (h->ade_plane_max + kTpThreads / 32 - 1) / (kTpThreads / 32);
   return a;
 }
 
@@ -136,15 +144,19 @@ template <typename T>
 void tp_update(xfb_handle* h, TimeP tp, cudaStream_t st, Prof* pf) {
   const Compiled& c = h->c;
   const TpArgs<T> a = tp_args<T>(h, tp);
-  const dim3 grid(a.c.bp + (c.ny * a.c.ns + kTpThreads - 1) / kTpThreads, c.nx);
+  const dim3 grid(a.nblk, c.nx);
   prof_begin(h, pf, XFB_K_UPDATE_H);
   k_tp_h<T><<<grid, kTpThreads, 0, st>>>(a);
   prof_end(h, pf);
   prof_begin(h, pf, XFB_K_UPDATE_E);
-  k_tp_e<T><<<grid, kTpThreads, 0, st>>>(a);
-  if (h->ade_deferred && h->n_ade_runs > 0)
-    k_tp_ade<T><<<(h->n_ade_runs + 3) / 4, 128, 0, st>>>(a, grid_params<T>(h, h->live), ade_params<T>(h),
-                                                         static_cast<const int2*>(h->ade_runs), h->n_ade_runs);
+  const bool runs = h->ade_deferred && h->n_ade_runs > 0;
+  if (runs && tp_ade_inside(h)) {
+    const long long row = static_cast<long long>(c.nx) * a.nblk + static_cast<long long>(a.run_hi - a.run_lo) * a.nade;
+    k_tp_e<T, true><<<static_cast<unsigned>(row), kTpThreads, 0, st>>>(a);
+  } else {
+    k_tp_e<T, false><<<grid, kTpThreads, 0, st>>>(a);
+    if (runs) k_tp_ade<T><<<(h->n_ade_runs + 3) / 4, 128, 0, st>>>(a, h->n_ade_runs);
+  }
   prof_end(h, pf);
 }
 
