@@ -256,7 +256,9 @@ int xfb_set_wait_limit(xfb_handle* h, int polls);
 int xfb_timed_step(xfb_handle* h, long long n, double* ms);
 
 /* Kernel classes of one time step, for xfb_profile_kernels (XFB_K_AUX: the
- * per-step TFSF line values of the one-sweep 3-D step). */
+ * per-step TFSF line values of the one-sweep 3-D step; XFB_K_NF2FF: the records
+ * of a scene with an NF2FF, whose launch takes the probes too; XFB_K_PROBE: the
+ * probes of a scene without). */
 enum xfb_kernel_class {
   XFB_K_UPDATE_H = 0, XFB_K_AUX = 1, XFB_K_UPDATE_E = 2, XFB_K_NF2FF = 3, XFB_K_PROBE = 4,
   XFB_K_MOVIE = 5, XFB_K_STEP = 6, XFB_K_CORRECT = 7, XFB_K_COUNT = 8

@@ -28,8 +28,8 @@ MAX_POLES = 4
 FAR_FIELD_STATIC_MAX_ANGLES = 4096  # XFB_FAR_FIELD_STATIC_MAX_ANGLES
 BATCH_AUTO, BATCH_PER_STEP, BATCH_PERSISTENT = 0, 1, 2  # xfb_batch_set_launch
 K_UPDATE_H, K_AUX, K_UPDATE_E, K_NF2FF, K_PROBE, K_MOVIE, K_STEP, K_CORRECT, K_COUNT = range(9)
-KERNEL_NAMES = ("k_tp_h/k_h3/k_h2 (H half-step)", "k_tfsf_lines (TFSF line values of the step)", "k_tp_e/k_e3/k_e2 (E half-step)", "k_nf2ff",
-                "k_probe", "k_movie", "k_step3 (one-sweep H+E step)",
+KERNEL_NAMES = ("k_tp_h/k_h3/k_h2 (H half-step)", "k_tfsf_lines (TFSF line values of the step)", "k_tp_e/k_e3/k_e2 (E half-step)",
+                "k_records (NF2FF, with the probes)", "k_records (probes)", "k_movie", "k_step3 (one-sweep H+E step)",
                 "boundary corrections (plain CPML/TFSF launches; k_labc_apply of the learned boundary)")
 PATH_AUTO, PATH_SPLIT, PATH_FUSED, PATH_PLAIN = 0, 1, 2, 3
 COEFF_NATIVE, COEFF_FP16, COEFF_BF16 = 0, 1, 2

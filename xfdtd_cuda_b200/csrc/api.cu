@@ -302,8 +302,8 @@ int launches_per_step(const xfb_handle* h) {
   if (plain(h)) {
     int faces = 0;
     for (int f = 0; f < 6; ++f) faces += c.pml[f] > 0;
-    return 6 + 2 * faces + (c.tfsf_on ? 24 : 0) + (c.nf_on ? 1 : 0) + (c.td_on ? 2 : 0) + (c.probes.empty() ? 0 : 1) +
-           static_cast<int>(c.movies.size());
+    return 6 + 2 * faces + (c.tfsf_on ? 24 : 0) + (c.nf_on || c.td_on || !c.probes.empty() ? 1 : 0) +
+           (c.td_on ? 1 : 0) + static_cast<int>(c.movies.size());
   }
   int bulk = 2;  // H and E half-steps
   if (h->two_pass) {
@@ -314,7 +314,7 @@ int launches_per_step(const xfb_handle* h) {
                             (h->lines_on ? 1 : 0);  // k_tfsf_lines
   }
   if (h->tb_on) return 1;  // one blocked launch per tb_steps steps, probes recorded inside
-  return bulk + (c.nf_on ? 1 : 0) + (c.td_on ? 2 : 0) + (c.probes.empty() ? 0 : 1) +
+  return bulk + (c.nf_on || c.td_on || !c.probes.empty() ? 1 : 0) + (c.td_on ? 1 : 0) +
          static_cast<int>(c.movies.size());
 }
 
@@ -863,7 +863,7 @@ int xfb_nf2ff_face_shape(const xfb_handle* h, int face, int s[3]) {
   return XFB_OK;
 }
 
-// Accumulates the NF2FF surface samples still in the ring (k_nf2ff keeps the
+// Accumulates the NF2FF surface samples still in the ring (k_records keeps the
 // samples of up to kNfRing steps before it adds them), so the accumulators
 // hold every step taken.  Enqueued on the stream that steps the handle (the
 // batch's stream while a batch steps it); launches kernels only.

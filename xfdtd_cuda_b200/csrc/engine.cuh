@@ -958,8 +958,15 @@ template <typename T>
 void enqueue_records(xfb_handle* h, int parity, TimeP tp, cudaStream_t s, Prof* pf) {
   const Compiled& c = h->c;
   GridP<T> g = grid_params<T>(h, out_set(h, parity));
+  RecordP r{};
+  unsigned blocks = 0;
+  const bool td_on = c.td_on && h->td_nchunks > 0;
+  if (td_on) {
+    r.td = td_params(h);
+    blocks += r.td_blocks = static_cast<unsigned>(h->td_nchunks);
+  }
   if (c.nf_on) {
-    NfP nf{};
+    NfP& nf = r.nf;
     nf.nfreq = static_cast<int>(c.freqs.size());
     for (int q = 0; q < 6; ++q) nf.box[q] = c.nf[q];
     for (int q = 0; q < 7; ++q) nf.off[q] = h->nf_off[q];
@@ -970,21 +977,16 @@ void enqueue_records(xfb_handle* h, int parity, TimeP tp, cudaStream_t s, Prof* 
     nf.done = h->nf_done;
     nf.own_lo = own_lo(h);
     nf.own_hi = own_hi(h);
-    prof_begin(h, pf, XFB_K_NF2FF);
-    k_nf2ff<T><<<static_cast<unsigned>((h->nf_npts + 255) / 256), 256, 0, s>>>(g, nf, tp);
-    prof_end(h, pf);
-  }
-  if (c.td_on && h->td_nchunks > 0) {
-    const TdP td = td_params(h);
-    prof_begin(h, pf, XFB_K_NF2FF);
-    k_nftd_chunks<T><<<h->td_nchunks, kTdChunk, 0, s>>>(g, td, tp);
-    k_nftd_bins<<<(6 * td.span + 127) / 128, 128, 0, s>>>(td, tp);
-    prof_end(h, pf);
+    blocks += r.nf_blocks = static_cast<unsigned>((h->nf_npts + kTdChunk - 1) / kTdChunk);
   }
   if (!c.probes.empty() && !h->tb_on) {  // the blocked 2-D kernel records its own
-    ProbeP pr{static_cast<int>(c.probes.size()), h->probe_idx, h->probe_field, h->probe_out, c.total_steps};
-    prof_begin(h, pf, XFB_K_PROBE);
-    k_probe<T><<<(pr.n + 127) / 128, 128, 0, s>>>(g, pr, tp);
+    r.pr = {static_cast<int>(c.probes.size()), h->probe_idx, h->probe_field, h->probe_out, c.total_steps};
+    blocks += static_cast<unsigned>((r.pr.n + kTdChunk - 1) / kTdChunk);
+  }
+  if (blocks) {
+    prof_begin(h, pf, r.td_blocks + r.nf_blocks ? XFB_K_NF2FF : XFB_K_PROBE);
+    k_records<T><<<blocks, kTdChunk, 0, s>>>(g, r, tp);
+    if (td_on) k_nftd_bins<<<(6 * r.td.span + 127) / 128, 128, 0, s>>>(r.td, tp);
     prof_end(h, pf);
   }
   for (size_t m = 0; m < c.movies.size(); ++m) {

@@ -118,7 +118,7 @@ struct xfb_handle {
   double2* th = nullptr;
   int nf_off[7] = {};
   long long nf_npts = 0;
-  // time-domain NF2FF (k_nftd_chunks / k_nftd_bins)
+  // time-domain NF2FF (k_records / k_nftd_bins)
   void* td_ent = nullptr;     // int4 per point
   double* td_tsd = nullptr;   // delay in steps per point
   double* td_prev = nullptr;  // [2][td_n]

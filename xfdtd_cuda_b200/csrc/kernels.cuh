@@ -13,9 +13,9 @@
 //          (BasicUpdator3D::updateE, src/updator/basic_updator/basic_updator_3d.cu:10-34;
 //          TemplateADEUpdateScheme::updateE, src/include/updator/ade_updator/
 //          template_ade_update_scheme.cuh:17-85; correctE of the TFSF/PML correctors)
-//   k_nf2ff running DFT of the NF2FF surface currents
+//   k_records running DFT of the NF2FF surface currents
 //          (src/nf2ff/frequency_domain/nf2ff_frequency_domain.data.cu:80-232)
-//   k_probe / k_movie monitors (src/monitor/movie_monitor.cu:17-46)
+//   k_records / k_movie monitors (src/monitor/movie_monitor.cu:17-46)
 //
 // Arithmetic order.  Every update, correction and accumulation evaluates its
 // terms in the reference's order (eNext/hNext, update_scheme.cuh:27-63; the
@@ -872,8 +872,8 @@ __device__ __forceinline__ void nf_face_samples(const GridP<T>& g, int axis, lon
 }
 
 template <typename T>
-__global__ void k_nf2ff(GridP<T> g, NfP nf, TimeP tp) {
-  const long long pt = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void nf2ff_point(const GridP<T>& g, const NfP& nf, const TimeP& tp, unsigned block) {
+  const long long pt = static_cast<long long>(block) * blockDim.x + threadIdx.x;
   if (pt >= nf.npts) return;
   const long long t = cur_step(tp);
   int face = 0;
@@ -913,7 +913,7 @@ __global__ void k_nf2ff(GridP<T> g, NfP nf, TimeP tp) {
 // point's two bins are t + d0 + rel and t + d0 + rel + 1 with rel = 0 or 1
 // (the rounding of delay + off + t can carry into the next integer), so a
 // chunk's contributions fall into three bins per tangential component:
-// k_nftd_chunks sums them per chunk (warp shuffles, then the warps in
+// k_records sums them per chunk (warp shuffles, then the warps in
 // order), k_nftd_bins adds, for every (component, bin) of the step's window,
 // the chunk sums that land there, in chunk order.  Both levels have a fixed
 // order: the potentials are reproducible run to run.
@@ -935,8 +935,8 @@ struct TdP {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kTdChunk) k_nftd_chunks(GridP<T> g, TdP td, TimeP tp) {
-  const int4 ch = td.chunk[blockIdx.x];
+__device__ __forceinline__ void nftd_chunk(const GridP<T>& g, const TdP& td, const TimeP& tp, unsigned block) {
+  const int4 ch = td.chunk[block];
   const long long t = cur_step(tp);
   const int face = ch.z >> 1, kind = ch.z & 1, axis = face >> 1;
   const bool neg = (face & 1) == 0;
@@ -977,7 +977,7 @@ __global__ void __launch_bounds__(kTdChunk) k_nftd_chunks(GridP<T> g, TdP td, Ti
   if (threadIdx.x < 6) {
     double s = 0;
     for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) s += red[w][threadIdx.x];
-    td.part[static_cast<long long>(blockIdx.x) * 6 + threadIdx.x] = s;
+    td.part[static_cast<long long>(block) * 6 + threadIdx.x] = s;
   }
 }
 
@@ -1003,14 +1003,36 @@ struct ProbeP {
 };
 
 template <typename T>
-__global__ void k_probe(GridP<T> g, ProbeP pr, TimeP tp) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void probe_value(const GridP<T>& g, const ProbeP& pr, const TimeP& tp, unsigned block) {
+  const int p = block * blockDim.x + threadIdx.x;
   if (p >= pr.n) return;
   const long long t = cur_step(tp);
   const int fld = pr.field[p];
   if (fld < 0) return;  // a probe of another x slab
   const T* f[6] = {g.ex, g.ey, g.ez, g.hx, g.hy, g.hz};
   pr.out[p * pr.total_steps + t] = static_cast<double>(f[fld][pr.idx[p]]);
+}
+
+// The records of a step in one launch of kTdChunk threads a block:
+// time-domain NF2FF chunks, then NF2FF points, then probes.  Each is a few
+// microseconds of dependent loads on small grids (step counter, index, field),
+// so apart they add up.  us per step as launches of their own and in one:
+// 36x32x40 FP64 16.8 and 14.9, 80x72x88 FP32 21.2 and 18.6, 156^3 FP32 69.5 and
+// 65.3 (NF2FF and probes), 106x100x117 FP64 93 and 89 (time-domain NF2FF, probes).
+struct RecordP {
+  TdP td;
+  NfP nf;
+  ProbeP pr;
+  unsigned td_blocks, nf_blocks;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kTdChunk) k_records(const __grid_constant__ GridP<T> g, const __grid_constant__ RecordP r,
+                                                      TimeP tp) {
+  const unsigned b = blockIdx.x;
+  if (b < r.td_blocks) nftd_chunk(g, r.td, tp, b);
+  else if (b < r.td_blocks + r.nf_blocks) nf2ff_point(g, r.nf, tp, b - r.td_blocks);
+  else probe_value(g, r.pr, tp, b - r.td_blocks - r.nf_blocks);
 }
 
 // Movie frame: copies the component box every `interval` steps
