@@ -589,6 +589,8 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
 #pragma unroll
         for (int q = 0; q < R * C; ++q)
           if (q == o) v = fld == XFB_EZ ? E[q / C][q % C] : fld == XFB_HX ? HX[q / C][q % C] : HY[q / C][q % C];
+        // H on the upper walls, which no step writes: not the lane's, updated past the grid
+        if (fld != XFB_EZ && (i0 + o / C >= nx || j0 + o % C >= ny)) v = (fld == XFB_HX ? s.hx : s.hy)[pr.idx[p]];
         pr.out[p * pr.total_steps + t0 + st] = static_cast<double>(v);
       }
     }
