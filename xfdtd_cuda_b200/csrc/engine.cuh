@@ -276,6 +276,7 @@ int init_device(xfb_handle* h) {
     if ((rc = copy(h, p, fld.data(), n * sizeof(int), cudaMemcpyHostToDevice))) return rc;
     if ((rc = alloc(h, &p, n * std::max(1LL, c.total_steps) * sizeof(double), true))) return rc;
     h->probe_out = static_cast<double*>(p);
+    if (h->tb_on && (rc = alloc(h, &h->probe_link, n * sizeof(int2), false))) return rc;
   }
   // movies
   for (const xfb_movie& mv : c.movies) {

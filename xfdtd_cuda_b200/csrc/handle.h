@@ -133,6 +133,7 @@ struct xfb_handle {
   long long* probe_idx = nullptr;
   int* probe_field = nullptr;
   double* probe_out = nullptr;
+  void* probe_link = nullptr;  // int2 per probe: scratch of the blocked 2-D kernel
   std::vector<double*> movie_out;
   std::vector<long long> movie_frames;
   long long* t_dev = nullptr;

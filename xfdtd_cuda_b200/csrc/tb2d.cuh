@@ -198,7 +198,7 @@ __device__ __forceinline__ void tb_add_col(T (&f)[kTbC], int c, double inc, doub
 template <typename T>
 __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
     k_step2_tb(GridP<T> s, GridP<T> d, PmlP<T> pm, PsiH<T> ps, PsiH<T> pd, const T* ezx_r, const T* ezy_r, T* ezx_w,
-               T* ezy_w, TfsfP tf_in, TimeP tp, ProbeP pr, int S, int n_mat, int nsx, int nsy) {
+               T* ezy_w, TfsfP tf_in, TimeP tp, ProbeP pr, int2* link, int S, int n_mat, int nsx, int nsy) {
   constexpr int R = kTbRows<T>, C = kTbC;
   extern __shared__ __align__(16) unsigned char tb_smem[];
   const int nw = blockDim.x >> 5, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -332,15 +332,32 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
   const bool tfr = tf_cols && tf.js < je_ && tf.je >= jb &&
                    ((i0 <= tf.is && il >= tf.is - 1) || (i0 <= tf.ie && il >= tf.ie));
   const bool tfc = tf_rows && i0 <= tf.ie && il >= tf.is;
-  bool probes = false;  // a probe of the interior in this lane's block
-  auto probe_at = [&](int p) {
-    const int i = static_cast<int>(pr.idx[p] / sx), j = static_cast<int>(pr.idx[p] - i * sx);
-    const bool own_i = i >= I0 && (i < I0 + geo.ti || I0 + geo.ti >= nx);
-    const bool own_j = j >= J0 && (j < J0 + geo.tj || J0 + geo.tj >= ny);
-    const bool here = own_i && own_j && i >= i0 && i <= il && j >= j0 && j < j0 + C;
-    return here && pr.field[p] >= 0 ? (i - i0) * C + j - j0 : -1;
-  };
-  for (int p = 0; p < pr.n; ++p) probes = probes || probe_at(p) >= 0;
+  // Probes of the interior (and of the wall nodes past the last tiles): every
+  // thread looks through its share of the list once per launch and puts the
+  // tile's probes on the chains of the lanes that hold them, {next, node and
+  // component} in `link`, heads in shared memory; at every step a lane walks its
+  // own chain.  With every lane searching the whole list, 600 probes on 320 x 220
+  // cells took 163 us per step (FP32; now 5.2, none 4.4) and 8 took 5.6 (4.6); on
+  // 1044^2 cells 600 took 184 (6.9).
+  int* heads = reinterpret_cast<int*>(tb_smem + lay.bytes);
+  if (pr.n > 0) {
+    heads[tid] = -1;
+    __syncthreads();
+    for (int p = tid; p < pr.n; p += blockDim.x) {
+      const int i = static_cast<int>(pr.idx[p] / sx), j = static_cast<int>(pr.idx[p] - i * sx), fld = pr.field[p];
+      const bool own_i = i >= I0 && (i < I0 + geo.ti || I0 + geo.ti >= nx);
+      const bool own_j = j >= J0 && (j < J0 + geo.tj || J0 + geo.tj >= ny);
+      if (fld < 0 || !own_i || !own_j) continue;
+      // H on the upper walls, which no step writes (the lanes' goes past the grid)
+      if (fld != XFB_EZ && (i >= nx || j >= ny)) {
+        const double v = static_cast<double>((fld == XFB_HX ? s.hx : s.hy)[pr.idx[p]]);
+        for (int st = 0; st < S; ++st) pr.out[p * pr.total_steps + t0 + st] = v;
+        continue;
+      }
+      const int w = (i - ib) / R, l = (j - jb) / C, o = (i - ib - w * R) * C + j - jb - l * C;
+      link[p] = make_int2(atomicExch(heads + 32 * w + l, p), o * 8 + fld);
+    }
+  }
 
   const int yr = yb.rank(lane);  // the lane's y-slab block, or -1
   // the lane's TFSF columns: js-1 and je for Hx, js and je for Ez
@@ -361,11 +378,14 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
 
   // warps without special cells: the plain update alone (their barriers are the
   // same CTA barrier as the other warps', so it is named)
-  const bool special = wall || pxw || tfr || tfc || !one || nyb > 0 || __any_sync(0xffffffffu, probes);
+  const bool special = wall || pxw || tfr || tfc || !one || nyb > 0 || (pr.n > 0 && __any_sync(0xffffffffu, heads[tid] >= 0));
   if (!special) {
     const int nt = blockDim.x;
     const T* xe_n = xe + min(warp + 1, nw - 1) * kTbCols + lane * C;  // (the last warp's rows past the region are not exact)
     const T* xh_p = xh + max(warp - 1, 0) * kTbCols + lane * C;
+    // (two steps per turn, the shuffles ahead of the barrier: in place, FP64 takes
+    // 18 register moves a step less; 2520^2 without probes 33.5 -> 32.6 us)
+#pragma unroll 2
     for (int st = 0; st < S; ++st) {
       tb_ld(nb, xe_n);
 #pragma unroll
@@ -379,11 +399,14 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
         }
       }
       tb_st(xh + warp * kTbCols + lane * C, HY[R - 1]);
+      T sd[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) sd[r] = __shfl_up_sync(0xffffffffu, HX[r][C - 1], 1);
       tb_sync(nt);
       tb_ld(nb, xh_p);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        const T hl = __shfl_up_sync(0xffffffffu, HX[r][C - 1], 1);
+        const T hl = sd[r];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           const T da = HX[r][c] - (c > 0 ? HX[r][(c + C - 1) % C] : hl);
@@ -581,17 +604,16 @@ __global__ void __launch_bounds__(32 * kTbMaxWarps<T>, 1)
         tb_str(col + geo.xi, p[1]);
       }
     }
-    if (probes) {  // record this lane's probes (and the wall nodes past the last tiles)
-      for (int p = 0; p < pr.n; ++p) {
-        const int o = probe_at(p), fld = pr.field[p];
-        if (o < 0) continue;
+    if (pr.n > 0) {
+      for (int p = heads[tid]; p >= 0;) {  // record this lane's probes
+        const int2 l = link[p];
+        const int o = l.y >> 3, fld = l.y & 7;
         T v = T(0);
 #pragma unroll
         for (int q = 0; q < R * C; ++q)
           if (q == o) v = fld == XFB_EZ ? E[q / C][q % C] : fld == XFB_HX ? HX[q / C][q % C] : HY[q / C][q % C];
-        // H on the upper walls, which no step writes: not the lane's, updated past the grid
-        if (fld != XFB_EZ && (i0 + o / C >= nx || j0 + o % C >= ny)) v = (fld == XFB_HX ? s.hx : s.hy)[pr.idx[p]];
         pr.out[p * pr.total_steps + t0 + st] = static_cast<double>(v);
+        p = l.x;
       }
     }
     tb_st(xe + warp * kTbCols + lane * C, E[0]);

@@ -23,7 +23,7 @@ void tb2d_slabs(const Compiled& c, int nw, int S, int& nsx, int& nsy) {
 template <typename T>
 size_t tb2d_bytes(const Compiled& c, int nw, int S, int& nsx, int& nsy) {
   tb2d_slabs<T>(c, nw, S, nsx, nsy);
-  return TbLayout<T>(nw, S, c.n_mat, nsx, nsy).bytes;
+  return TbLayout<T>(nw, S, c.n_mat, nsx, nsy).bytes + (c.probes.empty() ? 0 : 32 * nw * sizeof(int));  // the probes' heads
 }
 
 // Whether a scene takes the blocked step.  The second set of the E-side psi it
@@ -127,7 +127,7 @@ void launch_tb2d(xfb_handle* h, int off, int S) {
   k_step2_tb<T><<<grid, 32 * nw, smem, h->stream>>>(
       grid_params<T>(h, parity), grid_params<T>(h, 1 - parity), pml_params<T>(h), psi_h_set<T>(h, parity),
       psi_h_set<T>(h, 1 - parity), ez_x[parity], ez_y[parity], ez_x[1 - parity], ez_y[1 - parity], tfsf_params(h),
-      TimeP{h->t_dev, off}, pr, S, c.n_mat, nsx, nsy);
+      TimeP{h->t_dev, off}, pr, static_cast<int2*>(h->probe_link), S, c.n_mat, nsx, nsy);
 }
 
 // n steps as launches of odd step counts (each flips the sets once), as equal
