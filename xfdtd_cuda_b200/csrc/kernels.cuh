@@ -1165,13 +1165,84 @@ static __global__ void k_far(FarP fp) {
 // currents) instead of a sincos.  The currents are read at addresses uniform
 // over the lanes (one 16-byte broadcast per current), each once per 32
 // directions, which leaves the FP64 pipe as the bound.  The warps' sums are
-// added in warp order: results do not depend on the launch.  64800 directions
-// over 83 K points: 17.4 ms (k_far 54), FP64 pipe 36 % busy, the uniform loads'
+// added in warp order: results do not depend on the launch.  A call of 64800
+// directions over 83 K points takes 19.7 ms (with k_far 57); before the
+// compensation below the kernel's FP64 pipe was 36 % busy, the uniform loads'
 // wavefronts 55 %.
+//
+// A phase here serves a whole row or column and a sum a whole warp's rows, so
+// their errors average out over fewer terms than in k_far, where every point
+// has its own phase and 256 threads add: with arguments rounded at every
+// operation, a phase per face and plain sums the far field was 1.1 to 1.7 times
+// as far from an 80-bit one as k_far's.  Therefore the arguments carry what their
+// operations round off (far_proj, far_phase), a row's phase includes its face's,
+// and the sums of a column chunk are added and combined with their rounding errors
+// kept: 0.2 to 0.9 times k_far's error on boxes of 20 to 120 cells a side, 1 to 30
+// GHz at 1 mm, for 2 % more time.
 constexpr int kFarCols = 16, kFarWarps = 8;
 // directions from which k_far_many is used: 2048 make 64 CTAs; with fewer, its
 // CTAs of 32 directions leave most SMs idle, where k_far has one per direction
 constexpr int kFarManyMin = 2048;
+
+// a + b and its rounding error.
+__device__ __forceinline__ double far_add(double a, double b, double* e) {
+  const double s = __dadd_rn(a, b), t = __dsub_rn(s, a);
+  *e = __dadd_rn(__dsub_rn(a, __dsub_rn(s, t)), __dsub_rn(b, t));
+  return s;
+}
+
+// r x at x = o + m d (m exact), for a direction cosine r + rl; *e: what was rounded off.
+__device__ __forceinline__ double far_proj(double r, double rl, double o, double m, double d, double* e) {
+  const double p = __dmul_rn(m, d);
+  double xl;
+  const double x = far_add(o, p, &xl), q = __dmul_rn(r, x);
+  xl += fma(m, d, -p);
+  *e = fma(r, x, -q) + fma(r, xl, rl * x);
+  return q;
+}
+
+// cos and sin of k (q + ql).
+__device__ __forceinline__ void far_phase(double k, double q, double ql, double* s, double* c) {
+  const double a = __dmul_rn(k, q), al = fma(k, q, -a) + k * ql;
+  double sa, ca;
+  sincos(a, &sa, &ca);
+  *s = fma(al, ca, sa);
+  *c = fma(-al, sa, ca);
+}
+
+// far_combine of sums v + l, every rounding error kept to the last operation.
+__device__ __forceinline__ void far_combine_kept(const FarP& fp, const double* v, const double* l, double st, double ct,
+                                                 double sp, double cp, double* out) {
+  // h + hl += (a + al) (b + bl)
+  auto madd = [](double a, double al, double b, double bl, double& h, double& hl) {
+    const double p = __dmul_rn(a, b);
+    double e;
+    h = far_add(h, p, &e);
+    hl += e + (fma(a, b, -p) + fma(a, bl, al * b));
+  };
+  const double th[3] = {ct * cp, ct * sp, -st}, ph[3] = {-sp, cp, 0};
+  const double thl[3] = {fma(ct, cp, -th[0]), fma(ct, sp, -th[1]), 0};
+  const double f4 = 4 * 3.14159265358979323846, f = fp.k / f4, fl = fma(-f, f4, fp.k) / f4;
+#pragma unroll
+  for (int im = 0; im < 2; ++im) {
+    double x = 0, xl = 0, y = 0, yl = 0, n = 0, nl = 0, m = 0, ml = 0;  // L_phi + eta N_theta, L_theta - eta N_phi; N_theta, N_phi
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      madd(v[2 * c + im], l[2 * c + im], th[c], thl[c], n, nl);
+      madd(v[2 * c + im], l[2 * c + im], ph[c], 0, m, ml);
+      madd(v[6 + 2 * c + im], l[6 + 2 * c + im], ph[c], 0, x, xl);
+      madd(v[6 + 2 * c + im], l[6 + 2 * c + im], th[c], thl[c], y, yl);
+    }
+    madd(fp.eta, 0, n, nl, x, xl);
+    madd(-fp.eta, 0, m, ml, y, yl);
+    // E_theta = -j f x; E_phi = j f y
+    const double ex = f * x, ey = f * y;
+    x = ex + (fma(f, x, -ex) + fma(f, xl, fl * x));
+    y = ey + (fma(f, y, -ey) + fma(f, yl, fl * y));
+    out[im ? 0 : 1] = im ? x : -x;
+    out[im ? 2 : 3] = im ? -y : y;
+  }
+}
 
 static __global__ void __launch_bounds__(32 * kFarWarps, 2) k_far_many(FarP fp, int n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1180,23 +1251,30 @@ static __global__ void __launch_bounds__(32 * kFarWarps, 2) k_far_many(FarP fp, 
   sincos(fp.theta[a], &st, &ct);
   sincos(fp.phi[a], &sp, &cp);
   const double r[3] = {st * cp, st * sp, ct};
-  __shared__ double red[kFarWarps][12][32];
-  double acc[12];  // N (x,y,z re/im), L (x,y,z re/im)
+  const double rl[3] = {fma(st, cp, -r[0]), fma(st, sp, -r[1]), 0};
+  // the warps' sums, N (x,y,z re/im) and L (x,y,z re/im), and their rounding errors
+  __shared__ double acc[kFarWarps][12][32], err[kFarWarps][12][32];
 #pragma unroll
-  for (int q = 0; q < 12; ++q) acc[q] = 0;
+  for (int q = 0; q < 12; ++q) acc[warp][q][lane] = err[warp][q][lane] = 0;
 #pragma unroll
   for (int face = 0; face < 6; ++face) {
     const int axis = face >> 1, pos = face & 1;
     const int ar = axis == 0 ? 1 : 0, ac = axis == 2 ? 1 : 2;  // row and column axes of the point order
     const int nr = fp.box[2 * ar + 1] - fp.box[2 * ar], nc = fp.box[2 * ac + 1] - fp.box[2 * ac];
-    const double xr = fp.origin[ar] + (fp.box[2 * ar] + 0.5) * fp.d[ar], xc = fp.origin[ac] + (fp.box[2 * ac] + 0.5) * fp.d[ac];
-    double S[8];  // sums of ja, jb, ma, mb times the in-face phase
-#pragma unroll
-    for (int q = 0; q < 8; ++q) S[q] = 0;
+    const double mr = fp.box[2 * ar] + 0.5, mc = fp.box[2 * ac] + 0.5, ds = fp.d[ar] * fp.d[ac];
+    double nl;
+    const double nq = far_proj(r[axis], rl[axis], fp.origin[axis], fp.box[2 * axis + pos], fp.d[axis], &nl);
     for (int c0 = 0; c0 < nc; c0 += kFarCols) {
       double pr[kFarCols], pi[kFarCols];
 #pragma unroll
-      for (int c = 0; c < kFarCols; ++c) sincos(fp.k * (r[ac] * (xc + (c0 + c) * fp.d[ac])), &pi[c], &pr[c]);
+      for (int c = 0; c < kFarCols; ++c) {
+        double e;
+        const double q = far_proj(r[ac], rl[ac], fp.origin[ac], mc + (c0 + c), fp.d[ac], &e);
+        far_phase(fp.k, q, e, &pi[c], &pr[c]);
+      }
+      double S[8];  // sums of ja, jb, ma, mb times the phase
+#pragma unroll
+      for (int q = 0; q < 8; ++q) S[q] = 0;
       for (int row = warp; row < nr; row += kFarWarps) {
         const double2* src = fp.acc + fp.off[face] + static_cast<long long>(row) * nc + c0;
         double t[8];
@@ -1215,39 +1293,39 @@ static __global__ void __launch_bounds__(32 * kFarWarps, 2) k_far_many(FarP fp, 
             }
           }
         }
-        double rs, rc;
-        sincos(fp.k * (r[ar] * (xr + row * fp.d[ar])), &rs, &rc);
+        double rs, rc, e, f;
+        const double q = far_proj(r[ar], rl[ar], fp.origin[ar], mr + row, fp.d[ar], &e), qn = far_add(q, nq, &f);
+        far_phase(fp.k, qn, e + f + nl, &rs, &rc);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           S[2 * w] = fma(t[2 * w], rc, fma(-t[2 * w + 1], rs, S[2 * w]));
           S[2 * w + 1] = fma(t[2 * w], rs, fma(t[2 * w + 1], rc, S[2 * w + 1]));
         }
       }
-    }
-    double ns, ncs;
-    sincos(fp.k * (r[axis] * (fp.origin[axis] + fp.box[2 * axis + pos] * fp.d[axis])), &ns, &ncs);
-    const double ds = fp.d[ar] * fp.d[ac];
-    ns *= ds;
-    ncs *= ds;
-    const int ca = (axis + 1) % 3, cb = (axis + 2) % 3;
+      const int ca = (axis + 1) % 3, cb = (axis + 2) % 3;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const int o = (w < 2 ? 0 : 6) + 2 * (w & 1 ? cb : ca);
-      acc[o] += S[2 * w] * ncs - S[2 * w + 1] * ns;
-      acc[o + 1] += S[2 * w] * ns + S[2 * w + 1] * ncs;
+      for (int q = 0; q < 8; ++q) {
+        const int o = (q < 4 ? 0 : 6) + 2 * (q & 2 ? cb : ca) + (q & 1);
+        double e;
+        acc[warp][o][lane] = far_add(acc[warp][o][lane], S[q] * ds, &e);
+        err[warp][o][lane] += e;
+      }
     }
   }
-#pragma unroll
-  for (int q = 0; q < 12; ++q) red[warp][q][lane] = acc[q];
   __syncthreads();
   if (warp == 0 && blockIdx.x * 32 + lane < n) {
+    double v[12], l[12];
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
-      double v = red[0][q][lane];
-      for (int w = 1; w < kFarWarps; ++w) v += red[w][q][lane];
-      acc[q] = v;
+      double e;
+      v[q] = acc[0][q][lane];
+      l[q] = err[0][q][lane];
+      for (int w = 1; w < kFarWarps; ++w) {
+        v[q] = far_add(v[q], acc[w][q][lane], &e);
+        l[q] += err[w][q][lane] + e;
+      }
     }
-    far_combine(fp, acc, st, ct, sp, cp, fp.out + 4LL * a);
+    far_combine_kept(fp, v, l, st, ct, sp, cp, fp.out + 4LL * a);
   }
 }
 
