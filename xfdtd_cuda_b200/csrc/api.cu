@@ -924,10 +924,33 @@ int xfb_read_nf2ff_all(xfb_handle* h, int freq, double* dst, size_t len, long lo
                                : read_bytes_t<float>(h, dst, src, n * sizeof(double2));
 }
 
+// Whether k_far_many takes n directions, from the two kernels' times (us).  Its
+// CTAs of 32 directions run side by side, one per SM up to 4736 directions and
+// two up to 9472, so a call of a few costs as much as one of thousands: per
+// column chunk of a face its phases, per eight rows of the chunk a step of the
+// warps.  k_far's time goes with directions x points.  Measured, k_far and
+// k_far_many (us, with the call): 124^3-cell box 2048 directions 1929 and 2494,
+// 4096 3776 and 2518; 52^3 2048 437 and 571, 4096 772 and 586; 196 x 4 x 196
+// 2048 1750 and 2184, 4096 3279 and 2212; 4 x 196 x 4, where most of a chunk's
+// columns are past the face, 4096 252 and 304, 32768 2260 and 2282; 2 x 2 x 296,
+// two rows for eight warps, 4096 215 and 500, 32768 2059 and 3182.
+static bool far_many(const FarP& fp, int n) {
+  double cols = 0, rows = 0;
+  for (int axis = 0; axis < 3; ++axis) {
+    const int ar = axis == 0 ? 1 : 0, ac = axis == 2 ? 1 : 2;
+    const int nr = fp.box[2 * ar + 1] - fp.box[2 * ar], nc = fp.box[2 * ac + 1] - fp.box[2 * ac];
+    const int chunks = std::max(1, (nc + kFarCols - 1) / kFarCols);
+    cols += 2 * chunks * 3.7;
+    rows += 2 * chunks * ((nr + kFarWarps - 1) / kFarWarps) * (0.92 + 0.13 * nc / chunks);
+  }
+  const double wave = n <= 148 * 32 ? 35 + cols + rows : 35 + 1.5 * cols + 1.15 * rows;
+  return 1.05 * wave * std::ceil(n / (148 * 64.0)) < n / 2048.0 * (42 + 0.0198 * fp.npts);
+}
+
 // The far-field integral of n directions; the kernel writes all 4 outputs of
 // every direction.
 static void launch_far(const FarP& fp, int n, cudaStream_t s) {
-  if (n >= kFarManyMin) k_far_many<<<(n + 31) / 32, 32 * kFarWarps, 0, s>>>(fp, n);
+  if (far_many(fp, n)) k_far_many<<<(n + 31) / 32, 32 * kFarWarps, 0, s>>>(fp, n);
   else k_far<<<n, 256, 0, s>>>(fp);
 }
 

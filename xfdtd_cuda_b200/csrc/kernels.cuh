@@ -1181,9 +1181,6 @@ static __global__ void k_far(FarP fp) {
 // 0.9 times k_far's error on boxes of 20 to 120 cells a side, 1 to 30 GHz at 1 mm,
 // for 1 % more time.
 constexpr int kFarCols = 16, kFarWarps = 8;
-// directions from which k_far_many is used: 2048 make 64 CTAs; with fewer, its
-// CTAs of 32 directions leave most SMs idle, where k_far has one per direction
-constexpr int kFarManyMin = 2048;
 
 // a + b and its rounding error.
 __device__ __forceinline__ double far_add(double a, double b, double* e) {
