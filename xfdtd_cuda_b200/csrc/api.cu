@@ -49,7 +49,7 @@ int cuda_err(xfb_handle* h, cudaError_t e, const char* what) {
 namespace {
 struct PinPool {
   std::mutex mu;
-  std::vector<void*> idle;
+  std::vector<void*> idle[2];
   int users = 0;
 };
 // never destroyed: a handle may outlive the static objects of the process
@@ -57,33 +57,33 @@ PinPool& pin_pool() {
   static PinPool* pool = new PinPool;
   return *pool;
 }
-void* pin_alloc() {
+void* pin_alloc(int size) {
   void* p = nullptr;
-  if (cudaHostAlloc(&p, kPinBytes, cudaHostAllocPortable) != cudaSuccess) {
+  if (cudaHostAlloc(&p, kPinBytes[size], cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
   return p;
 }
-void* pin_take() {
+void* pin_take(int size) {
   PinPool& pool = pin_pool();
   {
     std::lock_guard<std::mutex> lock(pool.mu);
-    if (!pool.idle.empty()) {
-      void* p = pool.idle.back();
-      pool.idle.pop_back();
+    if (!pool.idle[size].empty()) {
+      void* p = pool.idle[size].back();
+      pool.idle[size].pop_back();
       return p;
     }
   }
-  return pin_alloc();
+  return pin_alloc(size);
 }
-void pin_give(void* p) {
+void pin_give(void* p, int size) {
   if (!p) return;
   PinPool& pool = pin_pool();
   {
     std::lock_guard<std::mutex> lock(pool.mu);
-    if (pool.users > 0 && pool.idle.size() < kPinIdle) {
-      pool.idle.push_back(p);
+    if (pool.users > 0 && pool.idle[size].size() < kPinIdle[size]) {
+      pool.idle[size].push_back(p);
       return;
     }
   }
@@ -102,34 +102,36 @@ void pin_use(xfb_handle* h) {
 namespace {
 void pin_release(xfb_handle* h) {
   if (!h->pin_user) return;
-  std::vector<void*> drop;
+  std::vector<void*> drop[2];
   {
     PinPool& pool = pin_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
-    if (--pool.users == 0) drop.swap(pool.idle);
+    if (--pool.users == 0)
+      for (int size = 0; size < 2; ++size) drop[size].swap(pool.idle[size]);
   }
-  for (void* p : drop) cudaFreeHost(p);
+  for (auto& d : drop)
+    for (void* p : d) cudaFreeHost(p);
 }
 }  // namespace
 
-void pin_warm() {
+void pin_warm(int size) {
   size_t have;
   {
     PinPool& pool = pin_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
-    have = pool.idle.size();
+    have = pool.idle[size].size();
   }
-  for (; have < 2; ++have) pin_give(pin_alloc());
+  for (; have < 2; ++have) pin_give(pin_alloc(size), size);
 }
 
-PinnedPair::PinnedPair() {
-  p[0] = pin_take();
-  p[1] = p[0] ? pin_take() : nullptr;
+PinnedPair::PinnedPair(int size) : size(size) {
+  p[0] = pin_take(size);
+  p[1] = p[0] ? pin_take(size) : nullptr;
 }
 
 PinnedPair::~PinnedPair() {
-  pin_give(p[0]);
-  pin_give(p[1]);
+  pin_give(p[0], size);
+  pin_give(p[1], size);
 }
 
 namespace {
@@ -1494,7 +1496,9 @@ int xfb_batch_step(xfb_batch* b, long long n) {
   const int rc = b->prec == XFB_FP64 ? batch_run<double>(b, n) : batch_run<float>(b, n);
   if (rc == XFB_OK && n > 0) {  // the read-backs' staging, pinned while the device steps
     pin_use(b->hs[0]);
-    pin_warm();
+    int size = 0;
+    for (const xfb_handle* h : b->hs) size = std::max(size, pin_size(h));
+    pin_warm(size);
   }
   return rc;
 }

@@ -1164,7 +1164,7 @@ int run_steps(xfb_handle* h, long long n) {
   // failure leaves the read-back to its unstaged form)
   if (n > 0) {
     if (readback_buffers(h))
-      pin_warm();
+      pin_warm(pin_size(h));
     else
       h->err.clear();
   }
@@ -1220,7 +1220,7 @@ __global__ void k_gather_field(const T* src, T* dst, long long sx, long long sy,
 // allocation fails.
 inline bool readback_buffers(xfb_handle* h) {
   pin_use(h);
-  if (!h->rb_dev && alloc(h, &h->rb_dev, kPinBytes, false) != XFB_OK) return false;
+  if (!h->rb_dev && alloc(h, &h->rb_dev, kPinBytes[pin_size(h)], false) != XFB_OK) return false;
   for (cudaEvent_t& ev : h->rb_ev)
     if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
       ev = nullptr;
@@ -1231,7 +1231,7 @@ inline bool readback_buffers(xfb_handle* h) {
 }
 
 // Read-back of component f into the caller's double array.  Chunks of
-// kPinBytes are gathered on the device in the compute type, copied
+// a pinned buffer's size are gathered on the device in the compute type, copied
 // into pinned host buffer c & 1, and widened to double by host threads while
 // the device gathers and copies the next chunk.  The host-side gather below
 // runs when the read-back buffers cannot be allocated.
@@ -1241,9 +1241,9 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
   comp_shape(h->c, f, s);
   const long long total = static_cast<long long>(s[0]) * s[1] * s[2];
   if (total == 0) return XFB_OK;
-  PinnedPair pin;
+  PinnedPair pin(pin_size(h));
   if (pin.ok() && readback_buffers(h)) {
-    constexpr long long kReadChunk = kPinBytes / sizeof(T);
+    const long long kReadChunk = kPinBytes[pin.size] / sizeof(T);
     const T* src = static_cast<const T*>(field_ptr(h, cur_set(h), f));
     T* stage = static_cast<T*>(h->rb_dev);
     const long long nch = (total + kReadChunk - 1) / kReadChunk;
@@ -1289,7 +1289,7 @@ int read_field_t(xfb_handle* h, int f, double* dst) {
 template <typename T>
 int read_bytes_t(xfb_handle* h, void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return XFB_OK;
-  PinnedPair pin;
+  PinnedPair pin(pin_size(h));
   if (!pin.ok() || !readback_buffers(h)) {
     h->err.clear();
     XFB_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
@@ -1297,7 +1297,7 @@ int read_bytes_t(xfb_handle* h, void* dst, const void* src, size_t bytes) {
     h->d2h_bytes += static_cast<long long>(bytes);
     return XFB_OK;
   }
-  constexpr size_t chunk = kPinBytes;
+  const size_t chunk = kPinBytes[pin.size];
   const size_t nch = (bytes + chunk - 1) / chunk;
   auto enqueue = [&](size_t c) -> cudaError_t {
     const size_t o = c * chunk, n = std::min(chunk, bytes - o);

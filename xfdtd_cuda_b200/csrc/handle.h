@@ -23,23 +23,29 @@ struct Buf {
 };
 
 // Pinned staging buffers of the read-backs, shared by the handles of the
-// process: a read takes two and gives them back.  Pinning costs 0.5 ms per MB,
-// so a pair per handle of 16 MB (FP32) or 32 MB (FP64) buffers cost 17 and
-// 35 ms per run, and once more 4 or 7 ms to unpin; at 4 MB a chunk's copy
-// (75 us) still hides its launches.  At most kPinIdle unused buffers are kept,
-// none once the last handle that reads back is destroyed.
-constexpr size_t kPinBytes = 4u << 20;
-constexpr size_t kPinIdle = 4;
-void pin_warm();  // have two unused buffers, as far as they can be had
+// process: a read takes two and gives them back.  Two sizes: pinning costs 0.5 ms
+// per MB, so a pair per handle of 16 MB (FP32) or 32 MB (FP64) buffers cost 17 and
+// 35 ms per run, and once more 4 or 7 ms to unpin, while every chunk costs some
+// 65 us beside its copy (75 us for 4 MB): wake-up, host threads, their last one.
+// Handles whose fields are of kPinLarge bytes or more, whose runs hide the
+// pinning, take the large ones.  Reads into faulted memory with 16 / 32 MB, with
+// 4 and with 16 MB chunks (ms; 12 host threads): FP32 20 MB 1.2, 1.3, 1.2, 40 MB
+// 1.6, 2.0, 1.9, 271 MB 7.4, 9.8, 7.7; FP64 40 MB 1.5, 1.9, 1.5, 160 MB 4.3, 6.2,
+// 4.4, 512 MB 11.2, 18.1, 12.8.  At most kPinIdle unused buffers of a size are
+// kept, none once the last handle that reads back is destroyed.
+constexpr size_t kPinBytes[2] = {4u << 20, 16u << 20};
+constexpr size_t kPinIdle[2] = {4, 2};
+constexpr size_t kPinLarge = 32u << 20;
+void pin_warm(int size);  // have two unused buffers, as far as they can be had
 struct PinnedPair {
+  int size;
   void* p[2];
-  PinnedPair();
+  explicit PinnedPair(int size);
   ~PinnedPair();
   PinnedPair(const PinnedPair&) = delete;
   PinnedPair& operator=(const PinnedPair&) = delete;
   bool ok() const { return p[0] && p[1]; }
 };
-
 
 }  // namespace xfb
 
@@ -176,7 +182,7 @@ struct xfb_handle {
   bool labc_on = false;
   void* labc_w = nullptr;
   float* labc_hist = nullptr;
-  // field read-back (read_field_t): a device gather buffer of kPinBytes and
+  // field read-back (read_field_t): a device gather buffer of the handle's pinned buffers' size and
   // the events that mark each pinned buffer's chunk as copied (chunk c lands in
   // buffer c & 1 while the host widens chunk c - 1 to double); pin_user: the
   // handle counts among the staging pool's users
@@ -254,6 +260,9 @@ T* as(void* p) { return static_cast<T*>(p); }
 void free_device(xfb_handle* h);
 void keep_blocks(xfb_handle* h);
 void pin_use(xfb_handle* h);  // count the handle among the staging pool's users
+inline int pin_size(const xfb_handle* h) {
+  return static_cast<size_t>(h->elems) * h->esize >= kPinLarge ? 1 : 0;
+}
 void free_spare(xfb_handle* h);
 int alloc(xfb_handle* h, void** out, size_t bytes, bool state);
 // n zeroed buffers of `bytes` each (256-byte aligned) from one cudaMalloc.
