@@ -1673,8 +1673,9 @@ int batch_run(xfb_batch* b, long long n) {
   if (b->two_pass) {
     b->tile = 1;
     b->launch = XFB_BATCH_PER_STEP;
-    // a chunk's graph of at most some 2000 launches
-    const long long most = std::max<long long>(4, std::min<long long>(b->graph_steps, 1024 / static_cast<long long>(b->hs.size())));
+    long long launches = 0;
+    for (const xfb_handle* h : b->hs) launches += launches_per_step(h);
+    const long long most = batch_graph_steps(b->graph_steps, launches);
     while (n > 0) {
       const int chunk = static_cast<int>(std::min(n, most));
       if ((rc = batch_chunk<T>(b, chunk, b->tile, true, b->launch))) return rc;

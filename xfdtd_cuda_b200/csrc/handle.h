@@ -5,6 +5,7 @@
 #include <cuda.h>  // CUtensorMap
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -206,6 +207,12 @@ struct xfb_handle {
 // chunk of steps (k_step3_persist).  The handles stay owned by the caller;
 // the batch owns only its tables, stream, counters and graphs.
 constexpr int kBatchChains = 16;  // parallel chains of a batch's two-pass step, at most
+// Steps of one graph of a batch's two-pass step: at most kBatchGraphLaunches
+// kernels, or one step's where that has more.
+constexpr long long kBatchGraphLaunches = 4096;
+inline int batch_graph_steps(int graph_steps, long long launches_of_a_step) {
+  return static_cast<int>(std::max(1LL, std::min<long long>(graph_steps, kBatchGraphLaunches / std::max(1LL, launches_of_a_step))));
+}
 
 struct xfb_batch {
   std::vector<xfb_handle*> hs;
