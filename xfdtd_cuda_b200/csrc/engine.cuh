@@ -292,8 +292,6 @@ int init_device(xfb_handle* h) {
   h->t_dev = static_cast<long long*>(p);
   if ((rc = alloc(h, &p, sizeof(unsigned long long), false))) return rc;
   h->scratch_u64 = static_cast<unsigned long long*>(p);
-  if ((rc = alloc(h, &p, sizeof(int), false))) return rc;
-  h->scratch_err = static_cast<int*>(p);
   XFB_CUDA(h, cudaStreamSynchronize(h->stream));
   return XFB_OK;
 }

@@ -145,7 +145,6 @@ struct xfb_handle {
   std::vector<long long> movie_frames;
   long long* t_dev = nullptr;
   unsigned long long* scratch_u64 = nullptr;
-  int* scratch_err = nullptr;  // blocked 2-D kernel: 2 when a tile's region outgrew its psi tables
   void* plain_c[18] = {};  // per-cell coefficient arrays of the plain path
   // one-sweep step work items per tile configuration
   // (int4: k tile | region kind << 16, j tile, first plane, end plane)
