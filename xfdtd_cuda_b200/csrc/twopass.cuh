@@ -271,8 +271,8 @@ __device__ __noinline__ void tp_h_cells(const TpArgs<T>& a, int i, int j, int k0
   }
 }
 
-// E pass of one vector cell by cell: as tp_h_cells, and dispersive vectors when
-// no separate pass does the ADE recursion.
+// E pass of one vector cell by cell: as tp_h_cells, and (FP64) dispersive vectors
+// when no separate pass does the ADE recursion.
 template <typename T>
 __device__ __noinline__ void tp_e_cells(const TpArgs<T>& a, int i, int j, int k0) {
   const TfsfP tf = a.tf.on ? tfsf_at_step(a.tf, cur_step(a.tp)) : a.tf;
@@ -293,11 +293,13 @@ __device__ __noinline__ void tp_e_cells(const TpArgs<T>& a, int i, int j, int k0
     T ex = e_next(cf.c, ex_o, cf.z, d_ex_a, cf.y, d_ex_b);
     T ey = e_next(cf.c, ey_o, cf.x, d_ey_a, cf.z, d_ey_b);
     T ez = e_next(cf.c, ez_o, cf.y, d_ez_a, cf.x, d_ez_b);
-    if (ad.kind != kAdeNone && ad.mat[3 * m] != T(0)) {
-      const long long bi = static_cast<long long>(i - ad.b0) * ad.bsx + static_cast<long long>(j - ad.b2) * ad.bsy + (k - ad.b4);
-      if (upd_x) ex = ade_e(ad, 0, bi, m, ex_o, ex);
-      if (upd_y) ey = ade_e(ad, 1, bi, m, ey_o, ey);
-      if (upd_z) ez = ade_e(ad, 2, bi, m, ez_o, ez);
+    if constexpr (sizeof(T) == 8) {  // (such FP32 scenes stay on the one-sweep step: tp_mixed_rounding)
+      if (ad.kind != kAdeNone && ad.mat[3 * m] != T(0)) {
+        const long long bi = static_cast<long long>(i - ad.b0) * ad.bsx + static_cast<long long>(j - ad.b2) * ad.bsy + (k - ad.b4);
+        if (upd_x) ex = ade_e(ad, 0, bi, m, ex_o, ex);
+        if (upd_y) ey = ade_e(ad, 1, bi, m, ey_o, ey);
+        if (upd_z) ez = ade_e(ad, 2, bi, m, ez_o, ez);
+      }
     }
     if (tf.on) tfsf_e(tf, IncTables{tf}, i, j, k, ex, ey, ez);
     if (sxp >= 0) {
@@ -511,7 +513,7 @@ __global__ void __launch_bounds__(kTpThreads, kTpBlocks) k_tp_e(const __grid_con
   const int sxp = slab(i, a.nx, pm.L[0], pm.L[1]);
   const int syp = slab(j, a.ny, pm.L[2], pm.L[3]);
   const bool zsl = k0 < pm.L[4] || k0 + V > a.nz - pm.L[5];
-  // cells to leave as they are: dispersive ones of the runs
+  // cells to leave as they are: dispersive ones of the runs (a.ad: FP64 only, see tp_e_cells)
   unsigned keep = 0;
   bool inline_ade = false;
 #pragma unroll
