@@ -82,7 +82,7 @@ void pin_give(void* p, int size) {
   PinPool& pool = pin_pool();
   {
     std::lock_guard<std::mutex> lock(pool.mu);
-    if (pool.users > 0 && pool.idle[size].size() < kPinIdle[size]) {
+    if (pool.idle[size].size() < 2u * pool.users) {
       pool.idle[size].push_back(p);
       return;
     }
@@ -106,8 +106,12 @@ void pin_release(xfb_handle* h) {
   {
     PinPool& pool = pin_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
-    if (--pool.users == 0)
-      for (int size = 0; size < 2; ++size) drop[size].swap(pool.idle[size]);
+    --pool.users;
+    for (int size = 0; size < 2; ++size)
+      while (pool.idle[size].size() > 2u * pool.users) {
+        drop[size].push_back(pool.idle[size].back());
+        pool.idle[size].pop_back();
+      }
   }
   for (auto& d : drop)
     for (void* p : d) cudaFreeHost(p);

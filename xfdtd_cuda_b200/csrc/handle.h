@@ -32,10 +32,13 @@ struct Buf {
 // pinning, take the large ones.  Reads into faulted memory with 16 / 32 MB, with
 // 4 and with 16 MB chunks (ms; 12 host threads): FP32 20 MB 1.2, 1.3, 1.2, 40 MB
 // 1.6, 2.0, 1.9, 271 MB 7.4, 9.8, 7.7; FP64 40 MB 1.5, 1.9, 1.5, 160 MB 4.3, 6.2,
-// 4.4, 512 MB 11.2, 18.1, 12.8.  At most kPinIdle unused buffers of a size are
-// kept, none once the last handle that reads back is destroyed.
+// 4.4, 512 MB 11.2, 18.1, 12.8.  Buffers are made when none is idle, so there are
+// as many as reads ran at once; at most two per handle that reads back are kept
+// idle, none once the last such handle is destroyed.  (With four kept in all, 4 and
+// 8 threads reading a handle each pinned and unpinned buffers at every read: 1 MB
+// fields 7 and 16 ms a round instead of 0.7 and 1, 52 MB 17 and 36 instead of 9 and
+// 15.)
 constexpr size_t kPinBytes[2] = {4u << 20, 16u << 20};
-constexpr size_t kPinIdle[2] = {4, 2};
 constexpr size_t kPinLarge = 32u << 20;
 void pin_warm(int size);  // have two unused buffers, as far as they can be had
 struct PinnedPair {
