@@ -1166,7 +1166,7 @@ static __global__ void k_far(FarP fp) {
 // over the lanes (one 16-byte broadcast per current), each once per 32
 // directions, which leaves the FP64 pipe as the bound.  The warps' sums are
 // added in warp order: results do not depend on the launch.  A call of 64800
-// directions over 83 K points takes 19.6 ms (with k_far 57); before the
+// directions over 83 K points takes 19.4 ms (with k_far 57); before the
 // compensation below the kernel's FP64 pipe was 36 % busy, the uniform loads'
 // wavefronts 55 %.
 //
@@ -1176,10 +1176,10 @@ static __global__ void k_far(FarP fp) {
 // operation, a phase per face and plain sums the far field was 1.1 to 1.7 times
 // as far from an 80-bit one as k_far's.  Therefore the arguments carry what their
 // products round off (far_phase; a face's coordinate, which all its points share,
-// to the last bit: far_proj), a row's phase includes its face's, and the sums of
+// to the last bit: far_proj), a column's phase includes its face's, and the sums of
 // a column chunk are added and combined with their rounding errors kept: 0.2 to
 // 0.9 times k_far's error on boxes of 20 to 120 cells a side, 1 to 30 GHz at 1 mm,
-// for 1 % more time.
+// in the same time (19.3 ms without).
 constexpr int kFarCols = 16, kFarWarps = 8;
 
 // a + b and its rounding error.
@@ -1267,7 +1267,7 @@ static __global__ void __launch_bounds__(32 * kFarWarps, 2) k_far_many(FarP fp, 
 #pragma unroll
       for (int c = 0; c < kFarCols; ++c) {
         const double x = fma(mc + (c0 + c), fp.d[ac], fp.origin[ac]), q = __dmul_rn(r[ac], x);
-        far_phase(fp.k, q, fma(r[ac], x, -q) + rl[ac] * x, &pi[c], &pr[c]);
+        far_phase(fp.k, q + nq, fma(r[ac], x, -q) + fma(rl[ac], x, nl), &pi[c], &pr[c]);
       }
       double S[8];  // sums of ja, jb, ma, mb times the phase
 #pragma unroll
@@ -1292,7 +1292,7 @@ static __global__ void __launch_bounds__(32 * kFarWarps, 2) k_far_many(FarP fp, 
         }
         double rs, rc;
         const double x = fma(mr + row, fp.d[ar], fp.origin[ar]), q = __dmul_rn(r[ar], x);
-        far_phase(fp.k, q + nq, fma(r[ar], x, -q) + fma(rl[ar], x, nl), &rs, &rc);
+        far_phase(fp.k, q, fma(r[ar], x, -q) + rl[ar] * x, &rs, &rc);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           S[2 * w] = fma(t[2 * w], rc, fma(-t[2 * w + 1], rs, S[2 * w]));
