@@ -1,5 +1,5 @@
 """Length of a batch's step graphs, without a GPU: tests/host_batch_graph.cu is
-compiled against the engine's headers.  A graph holds at most 4096 kernels, or
+compiled against the engine's headers.  A graph holds at most 2048 kernels, or
 one step's where a step of all scenes has more, counted from the scenes' real
 launches (records, dispersive passes and movies among them)."""
 import subprocess
