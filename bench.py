@@ -538,7 +538,7 @@ def main():
     if not args.no_accuracy and world == 1:
         try:
             from xfdtd_cuda_b200 import accuracy as A
-            accuracy = {"what": "relative L2 of the FP32 one-sweep engine against the FP64 engine (bit-identical "
+            accuracy = {"what": "relative L2 of the FP32 engine against the FP64 engine (bit-identical "
                                 "to the CPU restatement) at full size, per output",
                         "dielectric_sphere_156cube_2400_steps": A.fp32_vs_fp64("dielectric", 2400, local),
                         "dispersive_sphere_408cube_6000_steps": A.fp32_vs_fp64("dispersive", 6000, local),

@@ -248,7 +248,9 @@ int xfb_sync(xfb_handle* h);
  * latency).  A wait that runs out lets the copies in flight land, ends its
  * work item and sets the handle's error flag instead of hanging the device.
  * This call sets the limit (after xfb_init; 0 makes every wait give up at
- * once, which tests use to exercise that path without a device fault). */
+ * once, which tests use to exercise that path without a device fault).  A scene
+ * on the two-pass step, which has no waits, moves to the one-sweep step with its
+ * state, until the next xfb_init. */
 int xfb_set_wait_limit(xfb_handle* h, int polls);
 
 /* Advance n steps bracketed by CUDA events on the handle's stream (after a
@@ -274,10 +276,14 @@ int xfb_set_kernel_path(xfb_handle* h, int path);
 /* 2-D TMz scenes on the one-sweep path: steps advanced per launch by the
  * temporally blocked kernel (each CTA advances its tile plus a halo of that
  * many cells in registers and records its probes every step), odd, at most 31;
- * by default the library chooses (up to 11); 0 launches once per step.  Scenes
- * with movie monitors, or whose tiles do not fit a CTA's shared memory at that
- * many steps, step once per launch.  Results are identical either way.  Before
- * xfb_init. */
+ * fewer where the tile would not hold that many.  By default the library chooses
+ * (up to 11); 0 launches once per step, as do scenes with movie monitors and
+ * scenes whose CPML is wide against the blocks: with S the given count (9 by
+ * default), no window of 95 - S columns, or of the rows of a block of 16 to 64
+ * (more rows on larger grids) and S + 1 more, may hold over 16 CPML cells.  (A slab
+ * of 17 cells exceeds it, and so do two slabs of 9 some 70 cells apart along y.
+ * The rule also decides the layout of a checkpoint.)  Results are identical
+ * either way.  Before xfb_init. */
 int xfb_set_temporal_block(xfb_handle* h, int steps);
 
 /* Storage trial of the update coefficients, no counterpart in the reference

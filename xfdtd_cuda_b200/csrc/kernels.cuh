@@ -327,17 +327,12 @@ __device__ __forceinline__ T ade_e(const AdeP<T>& a, int comp, long long bi, int
   return e_new;
 }
 
-// Deferred ADE update of one dispersive cell of the box after a one-sweep
-// step.  The step kernel stored the plain eNext value of every cell in `d`;
-// this applies the TemplateADEUpdateScheme::updateE recursion with E^n from
-// `s` (k_ade_box: one thread per box cell, k fastest; k_ade_runs: one thread
-// per dispersive cell).  All inputs of a cell (E^n, plain values, J, J_prev,
-// E_prev of the three components) are loaded before any update, so the loads
-// overlap; the arithmetic and its order are those of ade_e.  Valid only when
-// no dispersive cell also takes a TFSF or CPML correction, which the
-// reference applies after the ADE update.
-// ADE update of one dispersive cell of the box: E^n in `ec`, the plain eNext
-// values in `pl`, E^{n+1} to `d`.
+// ADE update of one dispersive cell of the box (the TemplateADEUpdateScheme::
+// updateE recursion): E^n in `ec`, the plain eNext values in `pl`, E^{n+1} to
+// `d`.  All inputs of a cell (J, J_prev, E_prev of the three components) are
+// loaded before any update, so the loads overlap; the arithmetic and its order
+// are those of ade_e.  Valid only when no dispersive cell also takes a TFSF or
+// CPML correction, which the reference applies after the ADE update.
 template <typename T, int MP = 4>  // MP: XFB_MAX_POLES, or fewer where ad.P is known to be at most that
 __device__ __forceinline__ void ade_cell(const GridP<T>& d, const AdeP<T>& ad, int i, int j, int k, long long idx,
                                          int m, const T (&ec)[3], const T (&pl)[3]) {
@@ -397,7 +392,9 @@ __device__ __forceinline__ void ade_cell(const GridP<T>& d, const AdeP<T>& ad, i
   }
 }
 
-// The cell after a one-sweep step: the plain values are in `d`, E^n in `s`.
+// The cell after a one-sweep step, which stored the plain eNext value of every
+// cell in `d`; E^n is in `s` (k_ade_box: one thread per box cell, k fastest;
+// k_ade_runs: one thread per dispersive cell).
 template <typename T>
 __device__ __forceinline__ void ade_box_cell(const GridP<T>& s, const GridP<T>& d, const AdeP<T>& ad, int i, int j,
                                              int k, long long idx, int m) {
@@ -1164,11 +1161,10 @@ static __global__ void k_far(FarP fp) {
 // row phase per row; a point then costs 16 FMA per direction (four complex
 // currents) instead of a sincos.  The currents are read at addresses uniform
 // over the lanes (one 16-byte broadcast per current), each once per 32
-// directions, which leaves the FP64 pipe as the bound.  The warps' sums are
-// added in warp order: results do not depend on the launch.  A call of 64800
-// directions over 83 K points takes 19.4 ms (with k_far 57); before the
-// compensation below the kernel's FP64 pipe was 36 % busy, the uniform loads'
-// wavefronts 55 %.
+// directions.  The warps' sums are added in warp order: results do not depend on
+// the launch.  A call of 64800 directions over 83 K points takes 19.4 ms (with
+// k_far 57): the uniform loads bound it (54 % of their wavefronts, four cycles of
+// every warp's nine between issues waiting for one); the FP64 pipe is 35 % busy.
 //
 // A phase here serves a whole row or column and a sum a whole warp's rows, so
 // their errors average out over fewer terms than in k_far, where every point

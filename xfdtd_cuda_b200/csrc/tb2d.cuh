@@ -17,11 +17,13 @@
 // each), with one CTA barrier per half-step.  The former tile in shared memory
 // (fields, material ids and 18-entry coefficients read per cell) issued about
 // 230 instructions per cell update, this one about 13 in warps without walls,
-// TFSF lines or CPML cells.  Measured (us per step, before and after): 1044^2
-// cylinder FP32 14.0 and 6.8, FP64 21.7 and 11.9; 1519 x 751 FP64 23.1 and
-// 13.9; 2020 x 1720 FP32 13.4.  What bounds it: the tiles along the CPML, whose
-// warps all run the special rows below, take three times the others' time, and
-// at 1044^2 the tiles make barely two waves.
+// TFSF lines or CPML cells.  Measured (us per step, before and after, as the plan
+// runs them): 1044^2 cylinder FP32 14.0 and 6.5, FP64 21.7 and 12.3; 1519 x 751
+// FP64 23.1 and 13.2; 2020 x 1720 FP32 (after) 11.6.  What bounds it: the tiles
+// along the CPML, whose warps all run the special rows below, take three times the
+// others' time, and at 1044^2 the tiles make barely two waves; in FP64 also the
+// register spills of those rows (424 bytes of loads per thread at the 128 registers
+// of 16 warps; FP32 12).
 //
 // A warp whose cells share one material keeps its coefficients in registers,
 // the others look them up per cell; what else its cells need (PEC walls, TFSF

@@ -70,8 +70,12 @@ bool tb2d_plan(xfb_handle* h) {
   // A grid that fills the GPU with the largest tiles takes them: its launches
   // are bound by issue slots, and the longest blocks lose more to their halo
   // than they save.  us per step with 16 warps and S = 5 / 7 / 9 / 11: FP32
-  // 1044^2 8.2 / 6.9 / 7.1 / 7.7, 2020 x 1720 - / 12.5 / 12.2 / 11.9; FP64
-  // 1519 x 751 14.2 / 13.6 / 14.1 / -, 2020 x 1720 - / 23.9 / 24.0 / -.
+  // 1044^2 7.5 / 6.5 / 6.6 / 6.7, 1521 x 753 7.7 / 6.9 / 7.0 / 7.5, 2020 x 1720
+  // 13.1 / 11.9 / 11.6 / 11.4; FP64 1044^2 12.8 / 12.3 / 12.8 / 13.9, 1521 x 753
+  // 13.7 / 13.3 / 13.8 / 14.7, 2020 x 1720 24.7 / 23.1 / 23.4 / 24.9.  Where the
+  // last wave of the 7-step tiles is nearly empty, longer blocks are better than
+  // this rule: FP32 900^2 6.5 at 7, 5.7 at 11, 1400 x 800 7.2 and 6.7, 1200^2 7.6
+  // and 7.4; FP64 900^2 11.4 and (9) 10.8.
   auto tiles_of = [&](const TbGeom<T>& g) {
     return std::ceil(static_cast<double>(c.nx) / g.ti) * std::ceil(static_cast<double>(c.ny) / g.tj);
   };

@@ -6,8 +6,8 @@
 // tile in flight, its CPML and TFSF items add dependent loads to every plane,
 // and nothing hides them (two CTAs, 18 warps, per SM).  Here a thread owns V
 // consecutive cells of one row (V = 4 FP32, 2 FP64): every operand is one
-// 16-byte load, all loads of a pass are independent and issued first, 24 warps
-// per SM cover their latency, and the CPML and TFSF corrections run in the
+// 16-byte load, all loads of a pass are independent and issued first, up to 24
+// warps per SM cover their latency, and the CPML and TFSF corrections run in the
 // few warps that hold such cells.  Updating in place keeps one field set
 // live, and the passes sweep the planes in opposite directions, so grids up to
 // the L2's size stay there from pass to pass.
@@ -24,13 +24,14 @@
 // those of the one-sweep step.
 //
 // What bounds it, measured on a B200 (us per step, with NF2FF and probes; the
-// one-sweep step before): 156^3 FP32 69 (149), FP64 122 (240); 80x72x88 FP32 21
-// (66); 36x32x40 FP64 17 (81); 128x152x136 Debye FP64 97 (244); 408^3
-// Drude-Lorentz FP32 1190 (1356).  At 408^3 the H pass moves 2.9 GB in 0.45 ms,
-// 85 % of the copy bandwidth with what L2 keeps; at 156^3 load latency
-// dominates (20 warps per SM, 4 TB/s of DRAM and 44 % L2 hits); below 0.5 M
-// cells the launches do.  Scenes without a CPML stay on the one-sweep step,
-// whose lean interior body reaches 82 % of its 12 T + 1 bytes (384^3: 0.52 ms).
+// one-sweep step before): 156^3 FP32 65 (149), FP64 118 (240); 80x72x88 FP32 18.6
+// (66); 36x32x40 FP64 14.9 (81); 128x152x136 Debye FP64 97 (244); 408^3
+// Drude-Lorentz FP32 1183 (1356).  At 408^3 the H pass moves 2.69 GB in 0.43 ms
+// and the E pass 2.64 in 0.42, 96 % of the copy bandwidth; at 280^3, with the
+// dispersive runs in the E pass, 5.9 and 5.0 TB/s with 47 % L2 hits and 21 warps
+// per SM (80 registers), where load latency shows; below that it dominates, and
+// below 0.5 M cells the launches do.  Scenes without a CPML stay on the one-sweep
+// step, whose lean interior body reaches 82 % of its 12 T + 1 bytes (384^3: 0.52 ms).
 #pragma once
 
 #include "fused3d.cuh"
